@@ -162,7 +162,7 @@ def prepare(case, seed):
     if kind == "ensemble":
         members = []
         for m, (ni, nj, nk) in enumerate(W.ensemble_sizes(case["members"], case["grids"], (32, 32, 8), (56, 56, 14))):
-            members.append(_kept(_two_phase(api.Context(0), ni, nj, nk, seed + 100 * m, mixed=True)))
+            members.append(_kept(_two_phase(api.Context(0), ni, nj, nk, seed + 100 * m, mixed=False)))
         return {"kind": kind, "members": members, "sims": [m["sim"] for m in members],
                 "dts": [m["dt"] for m in members]}
     ctx = api.Context(0)
@@ -240,7 +240,9 @@ def run(state):
     if kind == "ensemble":
         for s in state["sims"]:
             s.restore_state()
-        api.ensemble_step_batched(state["sims"], state["dts"], precision=1)
+        _, statuses = api.ensemble_step_batched(state["sims"], state["dts"], precision=1)
+        if statuses.any():
+            raise RuntimeError("an ensemble member failed: %s" % statuses)
         return [dict(zip(("p", "N", "S"), s.state())) for s in state["sims"]]
     sim = state["sim"]
     sim.restore_state()
