@@ -101,6 +101,14 @@ int32_t rsg_sweep_mode(void);
  * are sequential loops). */
 rsg_status rsg_sweep_plan_check(int32_t n, const int32_t* row_ptr, const int32_t* col, int32_t sweep, int32_t ctas,
                                 int64_t* stats, char* msg, int32_t msg_len);
+/* The same for the block walk of a sweep (the ILU(0) solves inside the Krylov
+ * solvers): plans it on the host and walks the plan, with every staged value
+ * overwritten as early as the GPU may overwrite it, against the sequential
+ * solve.  stats (4 values, may be NULL): blocks, steps of all blocks, most
+ * steps of one block, most terms of a row.  RSG_UNSUPPORTED: the pattern has
+ * no block walk (its solves run the level walks). */
+rsg_status rsg_block_walk_check(int32_t n, const int32_t* row_ptr, const int32_t* col, int32_t sweep, int64_t* stats,
+                                char* msg, int32_t msg_len);
 /* Number of kernels this context has launched so far. */
 int64_t rsg_context_kernel_launches(rsg_ctx* ctx);
 /* Waits for all work queued on the context's stream. */
@@ -171,14 +179,16 @@ rsg_status rsg_solver_setup(rsg_solver* s, rsg_csr* A);
  * solution on exit (host arrays of length n). */
 rsg_status rsg_solver_solve(rsg_solver* s, rsg_csr* A, const double* b, double* x, rsg_solve_info* info);
 /* Level-walk shape of an ILU(0) solver (no counterpart in the reference).
- * The ILU(0) triangular solves walk the levels on one thread-block cluster,
- * planned for 16 CTAs of 4 warps and for 8 CTAs of 8 warps; the first setup on
- * a pattern times both on the factors and keeps the faster per sweep and per
- * precision (the walk autotuner).  Every shape gives the same bits.
+ * The level walks of ILU(0) triangular solves (rsg_precond_apply, the batched
+ * solves, and the solvers' applies on patterns without a block walk) run on
+ * one thread-block cluster, planned for 16 CTAs of 4 warps and for 8 CTAs of
+ * 8 warps; where the solvers use them, the first setup on a pattern times
+ * both on the factors and keeps the faster per sweep and per precision (the
+ * walk autotuner).  Every shape gives the same bits.
  * rsg_solver_set_walk_shape(s, 16 or 8) fixes the shape, 0 returns to the
- * timed choice (applied at the next rsg_solver_setup); rsg_solver_walk_shapes
- * reports the clusters in use: FP64 lower, upper, FP32 lower, upper (0: no
- * cluster walk).  RSG_UNSUPPORTED for other preconditioners. */
+ * library's choice (applied at the next rsg_solver_setup);
+ * rsg_solver_walk_shapes reports the clusters: FP64 lower, upper, FP32 lower,
+ * upper (0: no cluster walk).  RSG_UNSUPPORTED for other preconditioners. */
 rsg_status rsg_solver_set_walk_shape(rsg_solver* s, int32_t ctas);
 rsg_status rsg_solver_walk_shapes(rsg_solver* s, int32_t* shapes);
 /* The same for a simulator's pressure solver. */

@@ -58,6 +58,7 @@ def _declare(L):
         "rsg_abi_version": (i32, []),
         "rsg_sweep_mode": (i32, []),
         "rsg_sweep_plan_check": (i32, [i32, P(i32), P(i32), i32, i32, P(i64), C.c_char_p, i32]),
+        "rsg_block_walk_check": (i32, [i32, P(i32), P(i32), i32, P(i64), C.c_char_p, i32]),
         "rsg_status_string": (C.c_char_p, [i32]),
         "rsg_context_create": (i32, [i32, PP()]),
         "rsg_context_destroy": (i32, [vp]),
@@ -341,12 +342,12 @@ class IterativeSolver:
         self.ctx.check(lib().rsg_solver_setup(self.h, A.h), "setMatrix")
 
     def set_walk_shape(self, ctas):
-        """ILU(0) level-walk cluster: 16 or 8 CTAs, 0 for the autotuner's timed
-        choice (applied at the next set_matrix)."""
+        """ILU(0) level-walk cluster: 16 or 8 CTAs, 0 for the library's choice
+        (applied at the next set_matrix)."""
         self.ctx.check(lib().rsg_solver_set_walk_shape(self.h, int(ctas)), "set_walk_shape")
 
     def walk_shapes(self):
-        """Clusters of the ILU(0) walks in use: FP64 lower, upper, FP32 lower,
+        """Clusters of the ILU(0) level walks: FP64 lower, upper, FP32 lower,
         upper (0: no cluster walk)."""
         v = np.zeros(4, np.int32)
         self.ctx.check(lib().rsg_solver_walk_shapes(self.h, abi.iptr(v)), "walk_shapes")

@@ -674,6 +674,7 @@ struct Solver {
     if (hist.size() < cap) hist.resize(cap);
     A.refresh_sell();
     init_state();
+    pc->begin_solve(method == RSG_FGMRES_MIXED);
     switch (method) {
       case RSG_CG: run_cg(A, b, x); break;
       case RSG_BICGSTAB: run_bicgstab(A, b, x); break;

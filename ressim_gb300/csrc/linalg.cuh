@@ -109,6 +109,8 @@ struct Precond {
   // x := M^{-1} b (x may be read as the starting iterate, as SSOR does)
   virtual void apply(const double* b, double* x, const int* active) = 0;
   virtual void trans_apply(const double* b, double* x, const int* active) = 0;
+  // called once before a solve's applies (f32: before its apply_f32 calls)
+  virtual void begin_solve(bool f32) {}
   // Preconditioner.apply with MTJ's rounding (the solvers' applies may fuse
   // multiply-adds)
   virtual void apply_exact(const double* b, double* x) { apply(b, x, nullptr); }

@@ -15,8 +15,10 @@
 #include <atomic>
 #include <mutex>
 #include <cstdlib>
+#include <future>
 #include <string>
 
+#include "blockwalk.cuh"
 #include "ring.cuh"
 
 namespace rsg {
@@ -207,7 +209,8 @@ __global__ void __launch_bounds__(256) k_sweep_pipelined(SweepArgs<T> a) {
   }
 }
 
-// RSG_SWEEP=pipelined switches the ring walks off; RSG_RING_CTAS=8 or 16
+// RSG_SWEEP=pipelined switches the ring and block walks off, RSG_SWEEP=ring
+// the block walks; RSG_RING_CTAS=8 or 16
 // plans them for that cluster shape only (8 CTAs of 8 warps, 16 of 4);
 // otherwise both are planned and the walk autotuner picks.
 static bool ring_enabled() {
@@ -215,6 +218,11 @@ static bool ring_enabled() {
     const char* e = getenv("RSG_SWEEP");
     return !(e && std::string(e) == "pipelined");
   }();
+  return on;
+}
+
+static bool block_walks_enabled() {
+  static const bool on = getenv("RSG_SWEEP") == nullptr;
   return on;
 }
 
@@ -578,6 +586,7 @@ static std::string check_ring(int n, const std::vector<int>& rp, const std::vect
 // ------------------------------------------------------------ planning ----
 // entries: 0 lower part, 1 upper part, 2 full row without the diagonal.
 // upper_levels: schedule by dependencies on higher rows (backward sweeps).
+// The push-ring schedules (lower or upper ILU parts only) are planned apart.
 static void build_plan(Csr& A, SweepPlan& P, bool upper_levels, int entries, bool with_diag) {
   const int n = A.n;
   const auto& rp = A.h_rowptr;
@@ -668,15 +677,6 @@ static void build_plan(Csr& A, SweepPlan& P, bool upper_levels, int entries, boo
         src[base[s] + 32 * k + lane] = q;
       }
     }
-  // push-ring schedules (lower or upper ILU parts only), for both cluster
-  // shapes unless RSG_RING_CTAS fixes one
-  HostRing H[2];
-  bool ring[2] = {false, false};
-  for (int v = 0; v < 2; ++v) {
-    const int C = v == 0 ? 16 : 8;
-    if (ring_ctas() != 0 && ring_ctas() != C) continue;
-    ring[v] = entries != 2 && plan_ring(n, rp, cl, dg, upper_levels, entries, C, RING_SMEM_MAX, H[v]);
-  }
   Context& ctx = *A.ctx;
   P.nlev = nlev;
   P.nslices = ns;
@@ -698,10 +698,35 @@ static void build_plan(Csr& A, SweepPlan& P, bool upper_levels, int entries, boo
   up(P.len, len);
   up(P.col, col);
   up(P.src, src);
+  for (RingPlan& G : P.rings) G.R = 0;
+  if (with_diag) {
+    P.diag_src.resize(dsrc.size());
+    P.diag.resize(dsrc.size());
+    P.diagf.resize(dsrc.size());
+    up(P.diag_src, dsrc);
+  }
+  ctx.sync();
+}
+
+// The push-ring schedule of an ILU sweep for one cluster shape (0: 16 CTAs, 1:
+// 8), unless RSG_RING_CTAS fixes the other.  C == 0: none.
+static HostRing host_ring(const Csr& A, bool upper, int shape) {
+  HostRing H;
+  const int C = shape == 0 ? 16 : 8;
+  if (ring_ctas() != 0 && ring_ctas() != C) return H;
+  if (!plan_ring(A.n, A.h_rowptr, A.h_col, A.h_diag, upper, upper ? 1 : 0, C, RING_SMEM_MAX, H)) H.C = 0;
+  return H;
+}
+
+static void upload_rings(Csr& A, SweepPlan& P, const HostRing (&H)[2], bool with_diag) {
+  Context& ctx = *A.ctx;
+  auto up = [&](auto& dst, const auto& v) {
+    RSG_CUDA(cudaMemcpyAsync(dst.get(), v.data(), sizeof(v[0]) * v.size(), cudaMemcpyHostToDevice, ctx.stream));
+  };
   for (int v = 0; v < 2; ++v) {
     RingPlan& G = P.rings[v];
     G.R = 0;
-    if (!ring[v]) continue;
+    if (!H[v].C) continue;
     const HostRing& Hv = H[v];
     G.C = Hv.C;
     G.nlev = Hv.nlev;
@@ -736,12 +761,6 @@ static void build_plan(Csr& A, SweepPlan& P, bool upper_levels, int entries, boo
   // until the autotuner has timed them: 16 CTAs where that schedule exists
   P.pick[0] = P.pick[1] = P.rings[0].R ? 0 : 1;
   P.tuned = false;
-  if (with_diag) {
-    P.diag_src.resize(dsrc.size());
-    P.diag.resize(dsrc.size());
-    P.diagf.resize(dsrc.size());
-    up(P.diag_src, dsrc);
-  }
   ctx.sync();
 }
 
@@ -751,38 +770,40 @@ __global__ void k_fill_one(int n, T* x) {
   if (i < n) x[i] = T(1);
 }
 
-static void plan_values(Context& ctx, SweepPlan& P, const double* csr_vals, bool with_diag, bool f32) {
+static void plan_values(Context& ctx, SweepPlan& P, const double* csr_vals, bool with_diag, bool f64, bool f32) {
   int64_t size = (int64_t)P.src.size();
-  RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(size, 256), 256, 0, size, P.src.get(), csr_vals,
-             P.val.get());
+  if (f64)
+    RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(size, 256), 256, 0, size, P.src.get(), csr_vals,
+               P.val.get());
   if (f32)
     RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<float>, blocks_for(size, 256), 256, 0, size, P.src.get(), csr_vals,
                P.valf.get());
   if (with_diag) {
     int64_t ds = (int64_t)P.diag_src.size();
-    RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(ds, 256), 256, 0, ds, P.diag_src.get(),
+    if (f64) RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(ds, 256), 256, 0, ds, P.diag_src.get(),
                csr_vals, P.diag.get());
     if (f32)
       RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<float>, blocks_for(ds, 256), 256, 0, ds, P.diag_src.get(),
                  csr_vals, P.diagf.get());
   }
   for (RingPlan& G : P.rings) {
-  if (!G.R) continue;
-  const int64_t gs = (int64_t)G.src.size();
-  RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(gs, 256), 256, 0, gs, G.src.get(), csr_vals,
-             G.val.get());
-  if (f32)
-    RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<float>, blocks_for(gs, 256), 256, 0, gs, G.src.get(), csr_vals,
-               G.valf.get());
-  if (with_diag) {
+    if (!G.R) continue;
+    const int64_t gs = (int64_t)G.src.size();
+    if (f64)
+      RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(gs, 256), 256, 0, gs, G.src.get(), csr_vals,
+                 G.val.get());
+    if (f32)
+      RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<float>, blocks_for(gs, 256), 256, 0, gs, G.src.get(), csr_vals,
+                 G.valf.get());
+    if (!with_diag) continue;
     const int64_t ds = (int64_t)G.diag_src.size();
-    RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(ds, 256), 256, 0, ds, G.diag_src.get(),
-               csr_vals, G.diag.get());
+    if (f64)
+      RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<double>, blocks_for(ds, 256), 256, 0, ds, G.diag_src.get(),
+                 csr_vals, G.diag.get());
     if (f32)
       RSG_LAUNCH(ctx, "plan_gather", k_plan_gather<float>, blocks_for(ds, 256), 256, 0, ds, G.diag_src.get(),
                  csr_vals, G.diagf.get());
   }
-}
 }
 
 // Cluster launch of a level walk; falls back to one launch per level when
@@ -957,6 +978,11 @@ struct ILUPrecond : Precond {
   Context* ctx;
   Csr* A = nullptr;
   SweepPlan Lp, Up;
+  // the solvers' applies: block walks of both triangles, when the pattern
+  // has them (walk64 / walk32: and the factor values suit them)
+  BlockWalkPair walk;
+  bool walk64 = false, walk32 = false, walk32_filled = false;
+  bool level64 = false, level32 = false;  // the level walks' copies hold the current factors
   DeviceBuffer<double> LU, y;
   DeviceBuffer<float> yf;
   DeviceBuffer<int> flag, upd_ptr, upd_l, upd_j;
@@ -969,6 +995,19 @@ struct ILUPrecond : Precond {
     for (int k = 0; k < M.n; ++k)
       if (M.h_diag[k] < 0)
         throw Error(RSG_MISSING_DIAGONAL, "Missing diagonal entry on row " + std::to_string(k + 1));
+    // The schedules are independent of one another and of the rest of the
+    // analysis: other host threads plan them meanwhile (large patterns only).
+    const auto how = M.nnz > 200000 ? std::launch::async : std::launch::deferred;
+    std::future<HostRing> rings[2][2];
+    for (int u = 0; u < 2; ++u)
+      for (int v = 0; v < 2; ++v) rings[u][v] = std::async(how, [&M, u, v] { return host_ring(M, u == 1, v); });
+    std::future<HostBlockWalk> walks[2];
+    for (int u = 0; u < 2; ++u)
+      walks[u] = std::async(how, [&M, u] {
+        HostBlockWalk H;
+        if (!block_walks_enabled() || !plan_block_walk(M.n, M.h_rowptr, M.h_col, M.h_diag, u == 1, H)) H.nblk = 0;
+        return H;
+      });
     // ILU.java:113-120 reads colind[l] one past the end of row k when the
     // scan of row k runs off its end; that read can update row k+1 or run
     // off the array.  Such patterns are rejected rather than reproduced.
@@ -1024,10 +1063,33 @@ struct ILUPrecond : Precond {
     }
     build_plan(M, Lp, false, 0, false);
     build_plan(M, Up, true, 1, true);
+    for (int u = 0; u < 2; ++u) {
+      const HostRing H[2] = {rings[u][0].get(), rings[u][1].get()};
+      upload_rings(M, u == 0 ? Lp : Up, H, u == 1);
+    }
+    const HostBlockWalk wl = walks[0].get(), wu = walks[1].get();
+    walk.plan(ctx, M.n, wl, wu);
     LU.resize(std::max(M.nnz, 1));
     y.resize(M.n);
     yf.resize(M.n);
-    flag.resize(1);
+    flag.resize(2);
+  }
+
+  // the shape asked for, or 16 CTAs, where the solvers do not run the walks and nothing is timed
+  void pick_shapes() {
+    for (SweepPlan* P : {&Lp, &Up})
+      for (int v = 0; v < 2; ++v)
+        if (P->rings[v].R && P->rings[v].C == (force_ctas ? force_ctas : 16)) P->pick[0] = P->pick[1] = v;
+  }
+  // The level walks' copies of the factor values, gathered when first needed
+  // (by Preconditioner.apply, the batched solves, and the solvers' applies
+  // where there is no block walk).
+  void level_values(bool f32) {
+    bool& have = f32 ? level32 : level64;
+    if (have) return;
+    plan_values(*ctx, Lp, LU.get(), false, !f32, f32);
+    plan_values(*ctx, Up, LU.get(), true, !f32, f32);
+    have = true;
   }
 
   void setup(Csr& M) override {
@@ -1038,7 +1100,7 @@ struct ILUPrecond : Precond {
     }
     // LU.set(A) then factor() (ILU.java:80-125)
     RSG_LAUNCH(*ctx, "ilu_copy", k_copy, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, M.val.get(), LU.get());
-    RSG_CUDA(cudaMemsetAsync(flag.get(), 0, sizeof(int), ctx->stream));
+    RSG_CUDA(cudaMemsetAsync(flag.get(), 0, 2 * sizeof(int), ctx->stream));
     FactorArgs fa{Lp.nlev,      Lp.level_slices.get(), Lp.row.get(), M.rowptr.get(), M.col.get(), M.diag.get(),
                   upd_ptr.get(), upd_l.get(),           upd_j.get(),  LU.get(),       flag.get()};
     if (!launch_cluster(*ctx, "ilu_factor", k_factor_cluster, fa)) {
@@ -1047,13 +1109,26 @@ struct ILUPrecond : Precond {
         RSG_LAUNCH(*ctx, "ilu_factor", k_factor_level, blocks_for(slots, 256), 256, 0, fa, l);
       }
     }
-    int h = 0;
-    RSG_CUDA(cudaMemcpyAsync(&h, flag.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    level64 = level32 = walk32_filled = false;
+    if (walk.planned) walk.values<double>(LU.get(), M.diag.get(), flag.get() + 1);
+    int h[2] = {0, 0};
+    RSG_CUDA(cudaMemcpyAsync(h, flag.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
-    if (h) throw Error(RSG_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(h));
-    plan_values(*ctx, Lp, LU.get(), false, true);
-    plan_values(*ctx, Up, LU.get(), true, true);
-    if (!Lp.tuned || !Up.tuned) tune_walks();
+    if (h[0]) throw Error(RSG_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(h[0]));
+    // a factor whose scaled rows overflow keeps the level walks, which divide last
+    walk64 = walk.planned && !(h[1] & 1);
+    walk32 = walk.planned && !(h[1] & 2);
+    if (walk64 && walk32) pick_shapes();
+    else if (!Lp.tuned || !Up.tuned) tune_walks();
+  }
+
+  void begin_solve(bool f32) override {
+    if (!f32 && walk64) walk.begin<double>();
+    if (f32 && walk32) {
+      walk.begin<float>();
+      if (!walk32_filled) walk.values<float>(LU.get(), A->diag.get(), nullptr);
+      walk32_filled = true;
+    }
   }
 
   // Walk autotuner: the first setup on a pattern times each sweep's ring
@@ -1064,6 +1139,8 @@ struct ILUPrecond : Precond {
   // replaces the timing by a fixed shape.
   int force_ctas = 0;
   void tune_walks() {
+    level_values(false);
+    level_values(true);
     const int n = A->n;
     DeviceBuffer<double> bd(n), xd(n);
     DeviceBuffer<float> bf(n), xf(n);
@@ -1128,6 +1205,11 @@ struct ILUPrecond : Precond {
   // the Krylov solvers' applies: FP64 rows summed with fused multiply-adds
   void apply(const double* b, double* x, const int* active) override {
     // L.solve(b, y); U.solve(y, x)
+    if (walk64) {
+      walk.apply<double>(b, x, active);
+      return;
+    }
+    level_values(false);
     run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr, 0.0,
                                           active);
     run_sweep<SW_ILU_UPPER, double, true>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr,
@@ -1135,11 +1217,17 @@ struct ILUPrecond : Precond {
   }
   // Preconditioner.apply as MTJ rounds it (ILU.java:64-70)
   void apply_exact(const double* b, double* x) override {
+    level_values(false);
     run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr, 0.0, nullptr);
     run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr, 0.0,
                                     nullptr);
   }
   void apply_f32(const float* b, float* x, const int* active) override {
+    if (walk32) {
+      walk.apply<float>(b, x, active);
+      return;
+    }
+    level_values(true);
     run_sweep<SW_ILU_LOWER, float, true>(*ctx, "ilu_lower_f32", Lp, Lp.valf.get(), nullptr, b, yf.get(), nullptr,
                                          0.0f, active);
     run_sweep<SW_ILU_UPPER, float, true>(*ctx, "ilu_upper_f32", Up, Up.valf.get(), Up.diagf.get(), yf.get(), x,
@@ -1198,8 +1286,8 @@ void ILUPrecond::trans_apply(const double* b, double* x, const int* active) {
   }
   RSG_LAUNCH(*ctx, "ilu_trans_gather", k_gather_vals, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, T.tsrc.get(),
              LU.get(), T.At.val.get());
-  plan_values(*ctx, T.Ut, T.At.val.get(), true, false);
-  plan_values(*ctx, T.Lt, T.At.val.get(), false, false);
+  plan_values(*ctx, T.Ut, T.At.val.get(), true, true, false);
+  plan_values(*ctx, T.Lt, T.At.val.get(), false, true, false);
   run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_trans_upper", T.Ut, T.Ut.val.get(), T.Ut.diag.get(), b, y.get(), nullptr,
                                   0.0, active);
   run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_trans_lower", T.Lt, T.Lt.val.get(), nullptr, y.get(), x, nullptr, 0.0,
@@ -1229,8 +1317,8 @@ struct SSORPrecond : Precond {
       pattern_id = M.rowptr.get();
     }
     // FP32 copies too: the mixed-precision solver smooths its FP32 AMG levels with them
-    plan_values(*ctx, Fp, M.val.get(), true, true);
-    plan_values(*ctx, Bp, M.val.get(), true, true);
+    plan_values(*ctx, Fp, M.val.get(), true, true, true);
+    plan_values(*ctx, Bp, M.val.get(), true, true, true);
   }
   void apply_f32(const float* b, float* x, const int* active) override {
     run_sweep<SW_SSOR_FWD, float>(*ctx, "ssor_fwd_f32", Fp, Fp.valf.get(), Fp.diagf.get(), b, x, xxf.get(),
@@ -1330,6 +1418,8 @@ bool ilu_walk_shape(Precond* p, int force, int* shapes) {
 bool ilu_ring_plans(Precond* p, int prefer, const RingPlan** lower, const RingPlan** upper) {
   auto* ilu = dynamic_cast<ILUPrecond*>(p);
   if (!ilu || !ilu->A) return false;
+  ilu->level_values(false);
+  ilu->level_values(true);
   for (int pass = 0; pass < 2; ++pass)
     for (int v = 0; v < 2; ++v)
       if (ilu->Lp.rings[v].R && ilu->Up.rings[v].R && (pass == 1 || ilu->Lp.rings[v].C == prefer)) {
