@@ -6,6 +6,7 @@
 #include <unordered_map>
 
 #include "blockwalk.cuh"
+#include "dataflow.cuh"
 
 namespace rsg {
 
@@ -377,45 +378,6 @@ struct BlockWalkArgs {
   int* err;
 };
 
-// The sentinel of a value not written yet: a NaN that arithmetic does not
-// produce; a result with just these bits is stored as another NaN.
-template <typename T>
-struct Sentinel;
-template <>
-struct Sentinel<double> {
-  using Bits = unsigned long long;
-  static constexpr Bits bits = 0xfff4dead5eed0badull;
-  static __device__ __forceinline__ Bits guard(double v) {  // a stored value is never the sentinel
-    const int hi = __double2hiint(v) == (int)(bits >> 32) ? 0x7ff80000 : __double2hiint(v);
-    return (Bits)(unsigned)hi << 32 | (unsigned)__double2loint(v);
-  }
-  static __device__ __forceinline__ double value(Bits b) { return __longlong_as_double((long long)b); }
-  static __device__ __forceinline__ Bits load(const double* p) {
-    Bits v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-  }
-  static __device__ __forceinline__ void store(double* p, Bits v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-  }
-};
-template <>
-struct Sentinel<float> {
-  using Bits = unsigned;
-  static constexpr Bits bits = 0xffd5eed1u;
-  static __device__ __forceinline__ Bits of(float v) { return __float_as_uint(v); }
-  static __device__ __forceinline__ Bits guard(float v) { return of(v) == bits ? 0x7fc00000u : of(v); }
-  static __device__ __forceinline__ float value(Bits b) { return __uint_as_float(b); }
-  static __device__ __forceinline__ Bits load(const float* p) {
-    Bits v;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-  }
-  static __device__ __forceinline__ void store(float* p, Bits v) {
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-  }
-};
-
 __device__ __forceinline__ unsigned bw_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 
 // One thread's copy of a contiguous piece (16-byte aligned and sized), counted
@@ -457,21 +419,6 @@ __device__ __forceinline__ bool bw_test(const unsigned long long* bar, unsigned 
       : "memory");
   return ok != 0;
 }
-// Nanoseconds a wait may take: far more than a walk, also among other
-// kernels' walks.
-constexpr unsigned long long BW_LIMIT_NS = 2000000000ull;
-__device__ __forceinline__ unsigned long long bw_clock() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-// Whether a wait is to be given up, asked now and then (start: 0 at first):
-// it has taken too long, or some other wait of the launch has.
-__device__ __forceinline__ bool bw_over(unsigned long long& start, int* err) {
-  const unsigned long long t = bw_clock();
-  if (!start) start = t;
-  return t - start > BW_LIMIT_NS || *(volatile int*)err;
-}
 // Waits for a phase, the whole warp together.  A wait that is given up goes
 // on with what is there, so that every warp ends; the walk is then reported
 // as failed.
@@ -485,7 +432,7 @@ __device__ __forceinline__ void bw_wait(const unsigned long long* bar, unsigned 
         : "r"(bw_addr(bar)), "r"(parity)
         : "memory");
     if (__all_sync(0xffffffffu, ok)) return;
-    if ((i & 255) == 0 && __any_sync(0xffffffffu, bw_over(start, err))) {
+    if ((i & 255) == 0 && __any_sync(0xffffffffu, wait_over(start, err))) {
       atomicCAS(err, 0, 1);
       return;
     }
@@ -816,7 +763,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
         unsigned long long start = 0;
         for (int i = 1; __any_sync(0xffffffffu, mine && v == S::bits); ++i) {
           if (mine && v == S::bits) v = S::load(p);
-          if ((i & 255) == 0 && __any_sync(0xffffffffu, bw_over(start, g.err))) {
+          if ((i & 255) == 0 && __any_sync(0xffffffffu, wait_over(start, g.err))) {
             atomicCAS(g.err, 0, 1 + s);
             break;
           }
@@ -858,12 +805,6 @@ __global__ void k_block_walk_values(int nslots, int W, const int* __restrict__ r
     o[k * 32] = (T)v;
   }
   if (UPPER && bad && flag) atomicOr(flag, bad);
-}
-
-template <typename T>
-__global__ void k_sentinel(int64_t n, T* x) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] = Sentinel<T>::value(Sentinel<T>::bits);
 }
 
 void upload(Context& ctx, BlockWalk& P, const HostBlockWalk& H, const HostBlockWalk* lower, int n) {

@@ -1,0 +1,67 @@
+// What kernels share whose blocks or warps hand values to one another through
+// global memory while they run: a value not written yet holds a sentinel, and
+// a reader polls the value itself.  One trip through L2 then both announces
+// and delivers it, and no fence is needed.
+#pragma once
+#include "common.cuh"
+
+namespace rsg {
+
+// The sentinel: a NaN that arithmetic does not produce; a result with just
+// these bits is stored as another NaN.
+template <typename T>
+struct Sentinel;
+template <>
+struct Sentinel<double> {
+  using Bits = unsigned long long;
+  static constexpr Bits bits = 0xfff4dead5eed0badull;
+  static __device__ __forceinline__ Bits guard(double v) {  // a stored value is never the sentinel
+    const int hi = __double2hiint(v) == (int)(bits >> 32) ? 0x7ff80000 : __double2hiint(v);
+    return (Bits)(unsigned)hi << 32 | (unsigned)__double2loint(v);
+  }
+  static __device__ __forceinline__ double value(Bits b) { return __longlong_as_double((long long)b); }
+  static __device__ __forceinline__ Bits load(const double* p) {
+    Bits v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(double* p, Bits v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+  }
+};
+template <>
+struct Sentinel<float> {
+  using Bits = unsigned;
+  static constexpr Bits bits = 0xffd5eed1u;
+  static __device__ __forceinline__ Bits of(float v) { return __float_as_uint(v); }
+  static __device__ __forceinline__ Bits guard(float v) { return of(v) == bits ? 0x7fc00000u : of(v); }
+  static __device__ __forceinline__ float value(Bits b) { return __uint_as_float(b); }
+  static __device__ __forceinline__ Bits load(const float* p) {
+    Bits v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(float* p, Bits v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  }
+};
+
+template <typename T>
+__global__ void k_sentinel(int64_t n, T* x) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) x[i] = Sentinel<T>::value(Sentinel<T>::bits);
+}
+
+// Nanoseconds a wait may take: far more than a kernel, also among others.
+constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
+
+// Whether a wait is to be given up, asked now and then (start: 0 at first):
+// it has taken too long, or some other wait has.
+__device__ __forceinline__ bool wait_over(unsigned long long& start, const int* err) {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  if (!start) start = t;
+  return t - start > WAIT_LIMIT_NS || *(const volatile int*)err;
+}
+
+}  // namespace rsg

@@ -46,6 +46,7 @@ struct RingPlan {
 struct SweepPlan {
   int nlev = 0, nslices = 0;
   std::vector<int> h_level_slices;  // nlev + 1 slice offsets
+  std::vector<int> h_order;         // rows by level, ascending within one
   DeviceBuffer<int> level_slices, slice_base, slice_width, row, len, col, src;
   DeviceBuffer<double> val;   // FP64 coefficients (gathered from CSR via src)
   DeviceBuffer<float> valf;   // FP32 copy for the mixed-precision inner solver

@@ -19,6 +19,7 @@
 #include <string>
 
 #include "blockwalk.cuh"
+#include "factor.cuh"
 #include "ring.cuh"
 
 namespace rsg {
@@ -245,7 +246,8 @@ __global__ void k_sweep_level(SweepArgs<T> a, int l) {
   if (row >= 0) sweep_row<KIND, T>(a, slot, row, s);
 }
 
-// ILU(0) factorisation, one thread per row, rows of a level in parallel.
+// ILU(0) factorisation of patterns with rows of more than 32 entries (others:
+// factor.cu), one thread per row, rows of a level in parallel.
 // Row k reads only rows of earlier levels (its lower neighbours), which are
 // final once the barrier of their level has passed.
 // The elimination of row k is a fixed program of the pattern: for every
@@ -678,6 +680,7 @@ static void build_plan(Csr& A, SweepPlan& P, bool upper_levels, int entries, boo
       }
     }
   Context& ctx = *A.ctx;
+  P.h_order = order;
   P.nlev = nlev;
   P.nslices = ns;
   P.h_level_slices = level_slices;
@@ -985,9 +988,50 @@ struct ILUPrecond : Precond {
   bool level64 = false, level32 = false;  // the level walks' copies hold the current factors
   DeviceBuffer<double> LU, y;
   DeviceBuffer<float> yf;
+  RowFactor rows;
   DeviceBuffer<int> flag, upd_ptr, upd_l, upd_j;
   const int* pattern_id = nullptr;
   explicit ILUPrecond(Context* c) : ctx(c) {}
+
+  // elimination program of the level-by-level factorisation (see FactorArgs)
+  void elimination_program(Csr& M) {
+    const auto& rp = M.h_rowptr;
+    const auto& cl = M.h_col;
+    std::vector<int> uptr(M.nnz + 1, 0), ul, uj;
+    ul.reserve((size_t)M.nnz * 4);
+    uj.reserve((size_t)M.nnz * 4);
+    for (int k = 0; k < M.n; ++k) {
+      const int r1 = rp[k + 1];
+      for (int i = rp[k]; i < M.h_diag[k]; ++i) {
+        const int index = cl[i];
+        int l = rp[k] + 1;
+        int cnt = 0;
+        for (int j = M.h_diag[index] + 1; j < rp[index + 1]; ++j) {
+          while (l < r1 && cl[l] < cl[j]) l++;
+          if (l < r1 && cl[l] == cl[j]) {
+            ul.push_back(l);
+            uj.push_back(j);
+            cnt++;
+          }
+        }
+        uptr[i + 1] = cnt;
+      }
+    }
+    for (int q = 0; q < M.nnz; ++q) uptr[q + 1] += uptr[q];
+    if (ul.size() > (size_t)INT32_MAX) throw Error(RSG_UNSUPPORTED, "ILU elimination program too large");
+    if (ul.empty()) {
+      ul.push_back(0);
+      uj.push_back(0);
+    }
+    upd_ptr.resize(M.nnz + 1);
+    upd_l.resize(ul.size());
+    upd_j.resize(uj.size());
+    RSG_CUDA(cudaMemcpyAsync(upd_ptr.get(), uptr.data(), sizeof(int) * uptr.size(), cudaMemcpyHostToDevice,
+                             ctx->stream));
+    RSG_CUDA(cudaMemcpyAsync(upd_l.get(), ul.data(), sizeof(int) * ul.size(), cudaMemcpyHostToDevice, ctx->stream));
+    RSG_CUDA(cudaMemcpyAsync(upd_j.get(), uj.data(), sizeof(int) * uj.size(), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->sync();
+  }
 
   void analyse(Csr& M) {
     const auto& rp = M.h_rowptr;
@@ -1024,45 +1068,9 @@ struct ILUPrecond : Precond {
           }
       }
     }
-    // elimination program (see FactorArgs)
-    {
-      std::vector<int> uptr(M.nnz + 1, 0), ul, uj;
-      ul.reserve((size_t)M.nnz * 4);
-      uj.reserve((size_t)M.nnz * 4);
-      for (int k = 0; k < M.n; ++k) {
-        const int r1 = rp[k + 1];
-        for (int i = rp[k]; i < M.h_diag[k]; ++i) {
-          const int index = cl[i];
-          int l = rp[k] + 1;
-          int cnt = 0;
-          for (int j = M.h_diag[index] + 1; j < rp[index + 1]; ++j) {
-            while (l < r1 && cl[l] < cl[j]) l++;
-            if (l < r1 && cl[l] == cl[j]) {
-              ul.push_back(l);
-              uj.push_back(j);
-              cnt++;
-            }
-          }
-          uptr[i + 1] = cnt;
-        }
-      }
-      for (int q = 0; q < M.nnz; ++q) uptr[q + 1] += uptr[q];
-      if (ul.size() > (size_t)INT32_MAX) throw Error(RSG_UNSUPPORTED, "ILU elimination program too large");
-      if (ul.empty()) {
-        ul.push_back(0);
-        uj.push_back(0);
-      }
-      upd_ptr.resize(M.nnz + 1);
-      upd_l.resize(ul.size());
-      upd_j.resize(uj.size());
-      RSG_CUDA(cudaMemcpyAsync(upd_ptr.get(), uptr.data(), sizeof(int) * uptr.size(), cudaMemcpyHostToDevice,
-                               ctx->stream));
-      RSG_CUDA(cudaMemcpyAsync(upd_l.get(), ul.data(), sizeof(int) * ul.size(), cudaMemcpyHostToDevice, ctx->stream));
-      RSG_CUDA(cudaMemcpyAsync(upd_j.get(), uj.data(), sizeof(int) * uj.size(), cudaMemcpyHostToDevice, ctx->stream));
-      ctx->sync();
-    }
     build_plan(M, Lp, false, 0, false);
     build_plan(M, Up, true, 1, true);
+    if (!rows.plan(M, Lp.h_order)) elimination_program(M);
     for (int u = 0; u < 2; ++u) {
       const HostRing H[2] = {rings[u][0].get(), rings[u][1].get()};
       upload_rings(M, u == 0 ? Lp : Up, H, u == 1);
@@ -1092,15 +1100,8 @@ struct ILUPrecond : Precond {
     have = true;
   }
 
-  void setup(Csr& M) override {
-    if (A != &M || pattern_id != M.rowptr.get()) {
-      analyse(M);
-      A = &M;
-      pattern_id = M.rowptr.get();
-    }
-    // LU.set(A) then factor() (ILU.java:80-125)
+  void factor_levels(Csr& M) {
     RSG_LAUNCH(*ctx, "ilu_copy", k_copy, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, M.val.get(), LU.get());
-    RSG_CUDA(cudaMemsetAsync(flag.get(), 0, 2 * sizeof(int), ctx->stream));
     FactorArgs fa{Lp.nlev,      Lp.level_slices.get(), Lp.row.get(), M.rowptr.get(), M.col.get(), M.diag.get(),
                   upd_ptr.get(), upd_l.get(),           upd_j.get(),  LU.get(),       flag.get()};
     if (!launch_cluster(*ctx, "ilu_factor", k_factor_cluster, fa)) {
@@ -1109,11 +1110,25 @@ struct ILUPrecond : Precond {
         RSG_LAUNCH(*ctx, "ilu_factor", k_factor_level, blocks_for(slots, 256), 256, 0, fa, l);
       }
     }
+  }
+
+  void setup(Csr& M) override {
+    if (A != &M || pattern_id != M.rowptr.get()) {
+      analyse(M);
+      A = &M;
+      pattern_id = M.rowptr.get();
+    }
+    // LU.set(A) then factor() (ILU.java:80-125)
+    RSG_CUDA(cudaMemsetAsync(flag.get(), 0, 2 * sizeof(int), ctx->stream));
+    if (rows.planned) rows.run(M, LU.get(), flag.get());
+    else factor_levels(M);
     level64 = level32 = walk32_filled = false;
     if (walk.planned) walk.values<double>(LU.get(), M.diag.get(), flag.get() + 1);
-    int h[2] = {0, 0};
+    int h[3] = {0, 0, 0};
     RSG_CUDA(cudaMemcpyAsync(h, flag.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    RSG_CUDA(cudaMemcpyAsync(h + 2, ctx->dev_err.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
+    if (h[2]) ctx->check_device_error();  // a wait between rows ran out
     if (h[0]) throw Error(RSG_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(h[0]));
     // a factor whose scaled rows overflow keeps the level walks, which divide last
     walk64 = walk.planned && !(h[1] & 1);
