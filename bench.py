@@ -514,9 +514,9 @@ def ensemble_leg(args):
       (the plain FP64 GPU path, the configuration's reference point);
     * concurrent: rsg_ensemble_step, members on their own streams from host
       threads;
-    * batched: rsg_ensemble_step_batched, all members' pressure solves in
-      one persistent launch per Newton iteration, FP64 ILU(0) walks;
-    * batched_mixed: the same launch with the mixed-precision solver (FP64
+    * batched: rsg_ensemble_step_batched, FP64 (each member here has its own
+      context, so each runs on its own stream);
+    * batched_mixed: the same call with the mixed-precision solver (FP64
       flexible GMRES around 10 FP32 BiCGstab + FP32 ILU(0) steps), with its
       largest pressure difference against the serial FP64 step.
     Wall time around each call (host-driven Newton loop included).  The

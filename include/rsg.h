@@ -588,15 +588,16 @@ rsg_status rsg_sim_create_cubic(rsg_ctx* ctx, rsg_mesh* mesh, const rsg_cubic_fl
  * No counterpart in the reference (RS runs one field per process). */
 rsg_status rsg_ensemble_step(int32_t count, rsg_sim* const* sims, const double* dt, int32_t max_concurrent,
                              rsg_step_info* infos, int32_t* statuses);
-/* Ensembles in lockstep: one time step of dt[i] on every member, with the
- * pressure solves of all members in ONE persistent launch per Newton
- * iteration.  Each member's Discretisation.solve(dt)
- * (numerics/Discretisation.java:208-225) runs as in rsg_sim_step: the
- * members assemble their Jacobians and factor their ILU(0) preconditioners on
- * their own streams, then one kernel of thread-block clusters takes the
- * members from a work queue and solves each pressure system completely
- * (BiCGstab, mtj/.../sparse/BiCGstab.java:65-116, with ILU(0)) through
- * per-member offsets, and each member updates its pressure and tests its
+/* Ensembles: one time step of dt[i] on every member, with the pressure solver
+ * that `precision` names.  Each member's Discretisation.solve(dt)
+ * (numerics/Discretisation.java:208-225) runs as in rsg_sim_step.  A member
+ * with a context of its own whose ILU(0) factors have block walks is stepped
+ * on its own stream, from one of up to as many host threads as the machine
+ * has.  The others go in lockstep: they assemble their Jacobians and factor
+ * their ILU(0) preconditioners, then ONE persistent kernel of thread-block
+ * clusters takes them from a work queue and solves each pressure system
+ * completely (BiCGstab, mtj/.../sparse/BiCGstab.java:65-116, with ILU(0))
+ * through per-member offsets, and each updates its pressure and tests its
  * Newton convergence; converged members leave the loop.  Members must use
  * RSG_BICGSTAB with RSG_PC_ILU.  precision 0: BiCGstab in FP64 with the
  * FP64 ILU(0) factors; 1: the mixed-precision solver of RSG_FGMRES_MIXED
@@ -614,7 +615,7 @@ rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const 
  * independent systems in ONE persistent launch: solvers[i] (RSG_BICGSTAB with
  * RSG_PC_ILU, set up with A[i] by rsg_solver_setup) solves A[i] x[i] = b[i]
  * from the initial guess x[i], host arrays as in rsg_solver_solve.  The
- * launch is the ensemble solver of rsg_ensemble_step_batched (precision as
+ * launch is the lockstep solver of rsg_ensemble_step_batched (precision as
  * there); statuses[i] and infos[i] report each system (MTJ's reasons;
  * RSG_UNSUPPORTED for another method or preconditioner; RSG_BAD_ARG for a
  * solver not set up with its matrix), x[i] is copied back either way, and

@@ -667,15 +667,17 @@ struct Solver {
     ctx->sync();
   }
 
-  void solve(Csr& A, const double* b, double* x, rsg_solve_info* info) {
+  // run: the method to run (its own unless an ensemble asks for the mixed-precision one)
+  void solve(Csr& A, const double* b, double* x, rsg_solve_info* info) { solve(A, b, x, info, method); }
+  void solve(Csr& A, const double* b, double* x, rsg_solve_info* info, int run) {
     if (setup_for != &A) throw Error(RSG_BAD_ARG, "rsg_solver_setup must be called with this matrix first");
     ensure(A.n);
     size_t cap = std::min<size_t>((size_t)maxIter * 2 + 64, (size_t)1 << 22);
     if (hist.size() < cap) hist.resize(cap);
     A.refresh_sell();
     init_state();
-    pc->begin_solve(method == RSG_FGMRES_MIXED);
-    switch (method) {
+    pc->begin_solve(run == RSG_FGMRES_MIXED);
+    switch (run) {
       case RSG_CG: run_cg(A, b, x); break;
       case RSG_BICGSTAB: run_bicgstab(A, b, x); break;
       case RSG_GMRES: run_gmres(A, b, x); break;
@@ -904,6 +906,12 @@ void solver_setup(Solver& s, Csr& A) {
 }
 
 void solver_solve(Solver& s, Csr& A, const double* b, double* x, rsg_solve_info* info) { s.solve(A, b, x, info); }
+void solver_solve_member(Solver& s, Csr& A, const double* b, double* x, int precision, rsg_solve_info* info) {
+  s.solve(A, b, x, info, precision ? RSG_FGMRES_MIXED : RSG_BICGSTAB);
+}
+bool solver_runs_alone(Solver& s, int precision) {
+  return s.method == RSG_BICGSTAB && s.pc_kind == RSG_PC_ILU && ilu_has_block_walks(s.pc.get(), precision != 0);
+}
 
 SolverView solver_view(Solver& s) {
   return SolverView{s.method, s.pc_kind, s.pc.get(), s.rtol, s.atol, s.dtol, s.maxIter, s.setup_for, s.ctx, s.restart, s.inner_iters, s.inner_rtol};

@@ -139,6 +139,11 @@ SolverPtr make_solver(Context* ctx, int method, int precond, double rtol, double
 void solver_setup(Solver& s, Csr& A);
 void solver_solve(Solver& s, Csr& A, const double* b, double* x, rsg_solve_info* info);
 void solver_set_inner(Solver& s, int iterations, double rtol);
+// An ensemble member's pressure solve on its own stream: whether its solver
+// (BiCGstab + ILU(0)) has block walks for the precision, and the solve
+// (precision 0: BiCGstab, 1: the mixed-precision method) as solver_solve.
+bool solver_runs_alone(Solver& s, int precision);
+void solver_solve_member(Solver& s, Csr& A, const double* b, double* x, int precision, rsg_solve_info* info);
 // what a solver was created with, and its preconditioner
 struct SolverView {
   int method, pc_kind;
@@ -170,6 +175,8 @@ void ensemble_solve(const std::vector<EnsSystem>& sys, int precision, std::vecto
 // setup, for clusters of `prefer` CTAs when planned, else the other shape
 // (false for other preconditioners or patterns without ring schedules)
 bool ilu_ring_plans(Precond* p, int prefer, const RingPlan** lower, const RingPlan** upper);
+// whether the solvers' applies of an ILU(0) preconditioner run block walks, after its setup
+bool ilu_has_block_walks(Precond* p, bool f32);
 // walk autotuner of an ILU(0) preconditioner: force >= 0 sets the cluster
 // shape (0: timed choice, 16 or 8 CTAs), applied at the next setup; shapes
 // (when given) receives the clusters in use: FP64 lower, upper, FP32 lower,

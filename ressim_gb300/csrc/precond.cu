@@ -1430,6 +1430,11 @@ bool ilu_walk_shape(Precond* p, int force, int* shapes) {
   return true;
 }
 
+bool ilu_has_block_walks(Precond* p, bool f32) {
+  auto* ilu = dynamic_cast<ILUPrecond*>(p);
+  return ilu && (f32 ? ilu->walk32 : ilu->walk64);
+}
+
 bool ilu_ring_plans(Precond* p, int prefer, const RingPlan** lower, const RingPlan** upper) {
   auto* ilu = dynamic_cast<ILUPrecond*>(p);
   if (!ilu || !ilu->A) return false;
