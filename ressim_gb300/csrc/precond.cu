@@ -21,6 +21,7 @@
 #include "blockwalk.cuh"
 #include "factor.cuh"
 #include "ring.cuh"
+#include "ssorflow.cuh"
 
 namespace rsg {
 
@@ -35,9 +36,7 @@ struct SweepArgs {
   const T* val;
   const T* diag;
   const T* b;
-  T* x;   // output / in-place vector
-  T* xx;  // SSOR half iterate
-  T omega;
+  T* x;
   const int* active;
 };
 
@@ -51,34 +50,13 @@ __device__ __forceinline__ void sweep_row(const SweepArgs<T>& a, int slot, int r
   const int base = a.slice_base[s] + (slot & 31);
   const int len = a.len[slot];
   T sum = 0;
-  if constexpr (KIND == SW_SSOR_FWD || KIND == SW_SSOR_BWD) {
-    // sigma over the full row without the diagonal, CSR order; lower
-    // columns read the half iterate xx, upper columns read x.
 #pragma unroll 4
-    for (int k = 0; k < len; ++k) {
-      int q = base + 32 * k;
-      int c = a.col[q];
-      T v = (c < row) ? ld_l2(a.xx + c) : ld_l2(a.x + c);
-      sum += a.val[q] * v;
-    }
-    T d = a.diag[slot];
-    T sigma = (a.b[row] - sum) / d;
-    if (KIND == SW_SSOR_FWD) {
-      T xo = ld_l2(a.x + row);
-      st_l2(a.xx + row, xo + a.omega * (sigma - xo));
-    } else {
-      T xh = ld_l2(a.xx + row);
-      st_l2(a.x + row, xh + a.omega * (sigma - xh));
-    }
-  } else {
-#pragma unroll 4
-    for (int k = 0; k < len; ++k) {
-      int q = base + 32 * k;
-      sum += a.val[q] * ld_l2(a.x + a.col[q]);
-    }
-    if (KIND == SW_ILU_LOWER) st_l2(a.x + row, a.b[row] - sum);
-    else st_l2(a.x + row, (a.b[row] - sum) / a.diag[slot]);
+  for (int k = 0; k < len; ++k) {
+    int q = base + 32 * k;
+    sum += a.val[q] * ld_l2(a.x + a.col[q]);
   }
+  if (KIND == SW_ILU_LOWER) st_l2(a.x + row, a.b[row] - sum);
+  else st_l2(a.x + row, (a.b[row] - sum) / a.diag[slot]);
 }
 
 // One cluster walks all levels.  Every CTA of the cluster evaluates the same
@@ -957,9 +935,9 @@ static bool launch_ring(Context& ctx, const char* name, const SweepPlan& P, cons
 // solvers' applies); otherwise every path rounds as MTJ does.
 template <int KIND, typename T, bool FMA = false>
 static void run_sweep(Context& ctx, const char* name, const SweepPlan& P, const T* val, const T* diag, const T* b,
-                      T* x, T* xx, T omega, const int* active) {
+                      T* x, const int* active) {
   SweepArgs<T> a{P.nlev, P.level_slices.get(), P.slice_base.get(), P.row.get(), P.len.get(), P.col.get(), val, diag,
-                 b, x, xx, omega, active};
+                 b, x, active};
   if constexpr (KIND == SW_ILU_LOWER || KIND == SW_ILU_UPPER) {
     const RingPlan& G = P.ring(sizeof(T) == 4 ? 1 : 0);
     const bool ring = launch_ring<KIND, T, FMA>(ctx, name, P, RingPick<T>::val(G),
@@ -1187,20 +1165,18 @@ struct ILUPrecond : Precond {
           if (prec == 0) {
             ms = time_ms([&] {
               if (lower)
-                run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_tune", Lp, Lp.val.get(), nullptr, bd.get(), xd.get(),
-                                                      nullptr, 0.0, nullptr);
+                run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_tune", Lp, Lp.val.get(), nullptr, bd.get(), xd.get(), nullptr);
               else
                 run_sweep<SW_ILU_UPPER, double, true>(*ctx, "ilu_tune", Up, Up.val.get(), Up.diag.get(), bd.get(),
-                                                      xd.get(), nullptr, 0.0, nullptr);
+                                                      xd.get(), nullptr);
             });
           } else {
             ms = time_ms([&] {
               if (lower)
-                run_sweep<SW_ILU_LOWER, float, true>(*ctx, "ilu_tune", Lp, Lp.valf.get(), nullptr, bf.get(), xf.get(),
-                                                     nullptr, 0.0f, nullptr);
+                run_sweep<SW_ILU_LOWER, float, true>(*ctx, "ilu_tune", Lp, Lp.valf.get(), nullptr, bf.get(), xf.get(), nullptr);
               else
                 run_sweep<SW_ILU_UPPER, float, true>(*ctx, "ilu_tune", Up, Up.valf.get(), Up.diagf.get(), bf.get(),
-                                                     xf.get(), nullptr, 0.0f, nullptr);
+                                                     xf.get(), nullptr);
             });
           }
           if (ms < best_ms) {
@@ -1225,17 +1201,14 @@ struct ILUPrecond : Precond {
       return;
     }
     level_values(false);
-    run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr, 0.0,
-                                          active);
-    run_sweep<SW_ILU_UPPER, double, true>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr,
-                                          0.0, active);
+    run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), active);
+    run_sweep<SW_ILU_UPPER, double, true>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, active);
   }
   // Preconditioner.apply as MTJ rounds it (ILU.java:64-70)
   void apply_exact(const double* b, double* x) override {
     level_values(false);
-    run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr, 0.0, nullptr);
-    run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr, 0.0,
-                                    nullptr);
+    run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr);
+    run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr);
   }
   void apply_f32(const float* b, float* x, const int* active) override {
     if (walk32) {
@@ -1243,10 +1216,8 @@ struct ILUPrecond : Precond {
       return;
     }
     level_values(true);
-    run_sweep<SW_ILU_LOWER, float, true>(*ctx, "ilu_lower_f32", Lp, Lp.valf.get(), nullptr, b, yf.get(), nullptr,
-                                         0.0f, active);
-    run_sweep<SW_ILU_UPPER, float, true>(*ctx, "ilu_upper_f32", Up, Up.valf.get(), Up.diagf.get(), yf.get(), x,
-                                         nullptr, 0.0f, active);
+    run_sweep<SW_ILU_LOWER, float, true>(*ctx, "ilu_lower_f32", Lp, Lp.valf.get(), nullptr, b, yf.get(), active);
+    run_sweep<SW_ILU_UPPER, float, true>(*ctx, "ilu_upper_f32", Up, Up.valf.get(), Up.diagf.get(), yf.get(), x, active);
   }
   void trans_apply(const double* b, double* x, const int* active) override;
 };
@@ -1303,10 +1274,8 @@ void ILUPrecond::trans_apply(const double* b, double* x, const int* active) {
              LU.get(), T.At.val.get());
   plan_values(*ctx, T.Ut, T.At.val.get(), true, true, false);
   plan_values(*ctx, T.Lt, T.At.val.get(), false, true, false);
-  run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_trans_upper", T.Ut, T.Ut.val.get(), T.Ut.diag.get(), b, y.get(), nullptr,
-                                  0.0, active);
-  run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_trans_lower", T.Lt, T.Lt.val.get(), nullptr, y.get(), x, nullptr, 0.0,
-                                  active);
+  run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_trans_upper", T.Ut, T.Ut.val.get(), T.Ut.diag.get(), b, y.get(), active);
+  run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_trans_lower", T.Lt, T.Lt.val.get(), nullptr, y.get(), x, active);
 }
 
 // --------------------------------------------------------------- SSOR ----
@@ -1315,6 +1284,7 @@ struct SSORPrecond : Precond {
   Csr* A = nullptr;
   const int* pattern_id = nullptr;
   SweepPlan Fp, Bp;
+  SsorFlow flow;
   DeviceBuffer<double> xx;
   DeviceBuffer<float> xxf;
   double omegaF = 1, omegaR = 1;
@@ -1326,6 +1296,7 @@ struct SSORPrecond : Precond {
         if (M.h_diag[k] < 0) throw Error(RSG_MISSING_DIAGONAL, "Missing diagonal on row " + std::to_string(k + 1));
       build_plan(M, Fp, false, 2, true);
       build_plan(M, Bp, true, 2, true);
+      flow.plan(M, Fp, Bp);
       xx.resize(M.n);
       xxf.resize(M.n);
       A = &M;
@@ -1334,26 +1305,17 @@ struct SSORPrecond : Precond {
     // FP32 copies too: the mixed-precision solver smooths its FP32 AMG levels with them
     plan_values(*ctx, Fp, M.val.get(), true, true, true);
     plan_values(*ctx, Bp, M.val.get(), true, true, true);
+    flow.values(M.val.get());
   }
-  void apply_f32(const float* b, float* x, const int* active) override {
-    run_sweep<SW_SSOR_FWD, float>(*ctx, "ssor_fwd_f32", Fp, Fp.valf.get(), Fp.diagf.get(), b, x, xxf.get(),
-                                  (float)omegaF, active);
-    if (!reverse) {
-      RSG_CUDA(cudaMemcpyAsync(x, xxf.get(), sizeof(float) * A->n, cudaMemcpyDeviceToDevice, ctx->stream));
-      return;
-    }
-    run_sweep<SW_SSOR_BWD, float>(*ctx, "ssor_bwd_f32", Bp, Bp.valf.get(), Bp.diagf.get(), b, x, xxf.get(),
-                                  (float)omegaR, active);
+  // SSOR.java:143-194; x holds the starting iterate
+  template <typename T>
+  void run(const T* b, T* x, T* half, const int* active) {
+    flow.sweep<T>(false, b, x, half, (T)omegaF, active);
+    if (reverse) flow.sweep<T>(true, b, half, x, (T)omegaR, active);
+    else RSG_CUDA(cudaMemcpyAsync(x, half, sizeof(T) * A->n, cudaMemcpyDeviceToDevice, ctx->stream));
   }
-  void apply(const double* b, double* x, const int* active) override {
-    // SSOR.java:143-194; x holds the starting iterate
-    run_sweep<SW_SSOR_FWD, double>(*ctx, "ssor_fwd", Fp, Fp.val.get(), Fp.diag.get(), b, x, xx.get(), omegaF, active);
-    if (!reverse) {
-      RSG_LAUNCH(*ctx, "ssor_copy", k_copy, blocks_for(A->n, 256), 256, 0, (int64_t)A->n, xx.get(), x);
-      return;
-    }
-    run_sweep<SW_SSOR_BWD, double>(*ctx, "ssor_bwd", Bp, Bp.val.get(), Bp.diag.get(), b, x, xx.get(), omegaR, active);
-  }
+  void apply_f32(const float* b, float* x, const int* active) override { run(b, x, xxf.get(), active); }
+  void apply(const double* b, double* x, const int* active) override { run(b, x, xx.get(), active); }
   void trans_apply(const double* b, double* x, const int* active) override { apply(b, x, active); }
 };
 

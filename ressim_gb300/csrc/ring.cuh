@@ -13,7 +13,7 @@ namespace rsg {
 
 namespace cg = cooperative_groups;
 
-enum SweepKind { SW_ILU_LOWER = 0, SW_ILU_UPPER = 1, SW_SSOR_FWD = 2, SW_SSOR_BWD = 3, SW_ILU_LOWER_T = 4 };
+enum SweepKind { SW_ILU_LOWER = 0, SW_ILU_UPPER = 1, SW_ILU_LOWER_T = 4 };
 
 // ILU sweeps on one thread-block cluster whose CTAs own contiguous blocks
 // of rows, with the computed values exchanged through distributed shared

@@ -1,0 +1,390 @@
+// SSOR sweeps (mtj/src/no/uib/cipr/matrix/sparse/SSOR.java:143-194) as a
+// dataflow of rows: a row starts as soon as the values it reads are there,
+// polling the values themselves (dataflow.cuh).  Rows are summed in CSR order,
+// products and sums rounded apart, as the Java loop does.
+//
+// What bounds a sweep is its chain of dependent rows (about 160 on a 40 x 36 x
+// 12 grid, and nearly as many rows on the narrow coarse levels of an AMG
+// hierarchy), so the values travel by the shortest way there is:
+//  * Patterns whose vector fits shared memory and whose rows have at most 32
+//    entries: one CTA, a thread per row, a warp per slice of 32 rows of one
+//    level (the sweep plan's SELL slices).  A hop is a poll of shared memory.
+//    A warp's slices are far apart in the order, so the loads of one pass
+//    behind the chain of the slices before it.
+//  * Wider rows (Galerkin products): a warp per row, a lane per entry, the
+//    lanes' products summed in order through shuffles.  One CTA while the
+//    rows are few; all SMs, with the values polled through L2, for more.
+// The V-cycle sweeps of a 40 x 36 x 12 system in FP32: 27 us on the 17,280
+// rows (slices) and 34 us on average on the three coarse levels (a warp per
+// row), against 245 us on average on one 8-CTA cluster with a barrier per
+// level.  That solve with its setup: 71 ms against 285.
+#include <mutex>
+
+#include "dataflow.cuh"
+#include "ssorflow.cuh"
+
+namespace rsg {
+
+namespace {
+
+constexpr int FLOW_WIDTH = 32;               // entries of a row held in registers (slices)
+constexpr int FLOW_GROUP = 8;                // operands polled together
+constexpr int FLOW_CHUNKS = 4;               // 32 entries each held in registers (rows)
+constexpr int FLOW_ROWS_MAX = 4096;          // rows one CTA takes a warp each: 100 instructions a row
+constexpr size_t FLOW_SMEM = 200 * 1024;
+template <typename T>
+constexpr int FLOW_THREADS = sizeof(T) == 4 ? 512 : 256;  // slices: two or four registers an entry
+constexpr int FLOW_ROW_THREADS = 512;
+
+// The values being computed, in the CTA's shared memory or in global memory.
+template <typename T, bool SMEM>
+struct Fresh;
+template <bool SMEM>
+struct Fresh<double, SMEM> {
+  using S = Sentinel<double>;
+  static __device__ __forceinline__ S::Bits load(const double* p) {
+    if (!SMEM) return S::load(p);
+    S::Bits v;
+    asm volatile("ld.relaxed.cta.shared.u64 %0, [%1];" : "=l"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(double* p, S::Bits v) {
+    if (!SMEM) return S::store(p, v);
+    asm volatile("st.relaxed.cta.shared.u64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "l"(v) : "memory");
+  }
+};
+template <bool SMEM>
+struct Fresh<float, SMEM> {
+  using S = Sentinel<float>;
+  static __device__ __forceinline__ S::Bits load(const float* p) {
+    if (!SMEM) return S::load(p);
+    S::Bits v;
+    asm volatile("ld.relaxed.cta.shared.u32 %0, [%1];" : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(float* p, S::Bits v) {
+    if (!SMEM) return S::store(p, v);
+    asm volatile("st.relaxed.cta.shared.u32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
+  }
+};
+
+__device__ __forceinline__ double from_bits(unsigned long long b) { return Sentinel<double>::value(b); }
+__device__ __forceinline__ float from_bits(unsigned b) { return Sentinel<float>::value(b); }
+
+template <typename T>
+struct SsorArgs {
+  int n;
+  const T* val;
+  const T* b;
+  const T* old;
+  T* out;
+  T omega;
+  const int* active;
+  int* err;
+  // slices
+  int nslices;
+  const int *slice_base, *row, *len, *scol;
+  const T* diag;
+  // rows
+  const int *order, *rowptr, *col, *dpos;
+  unsigned* ticket;
+};
+
+// Waits until none of a lane's operands u[k] with at[k] >= 0 is missing, the
+// warp together.  A wait given up goes on with what is there.
+template <typename T, bool SMEM, int N>
+__device__ __forceinline__ void await(typename Sentinel<T>::Bits (&u)[N], const int* at, const T* fresh, int row,
+                                      int* err) {
+  using S = Sentinel<T>;
+  unsigned long long start = 0;
+  for (int w = 1;; ++w) {
+    bool missing = false;
+#pragma unroll
+    for (int k = 0; k < N; ++k) missing |= at[k] >= 0 && u[k] == S::bits;
+    if (!__any_sync(0xffffffffu, missing)) return;
+    if ((w & 255) == 0 && __any_sync(0xffffffffu, wait_over(start, err))) {
+      atomicCAS(err, 0, 1 + max(row, 0));
+      return;
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (at[k] >= 0 && u[k] == S::bits) u[k] = Fresh<T, SMEM>::load(fresh + at[k]);
+  }
+}
+
+template <typename T, bool BWD>
+__global__ void __launch_bounds__(FLOW_THREADS<T>, 1) k_ssor_slices(SsorArgs<T> a) {
+  if (a.active && *a.active != 0) return;
+  using S = Sentinel<T>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  T* fresh = reinterpret_cast<T*>(smem);
+  for (int i = threadIdx.x; i < a.n; i += blockDim.x) fresh[i] = S::value(S::bits);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  // Slices in order, every nwarps-th a warp's: the first one not finished
+  // reads finished ones only, and its warp has no earlier one left.
+  struct Meta {
+    int row, len, base;
+  };
+  auto meta = [&](int s) {
+    Meta m{-1, 0, 0};
+    if (s < a.nslices) {
+      m.row = a.row[s * 32 + lane];
+      m.len = m.row >= 0 ? a.len[s * 32 + lane] : 0;
+      m.base = a.slice_base[s] + lane;
+    }
+    return m;
+  };
+  Meta next = meta(threadIdx.x >> 5);
+  for (int s = threadIdx.x >> 5; s < a.nslices; s += nwarps) {
+    const Meta m = next;
+    T v[FLOW_WIDTH];
+    int at[FLOW_WIDTH];
+    typename S::Bits u[FLOW_WIDTH / FLOW_GROUP][FLOW_GROUP];
+#pragma unroll
+    for (int k = 0; k < FLOW_WIDTH; ++k) {
+      at[k] = -1;
+      v[k] = 0;
+      if (k < m.len) {
+        at[k] = a.scol[m.base + 32 * k];
+        v[k] = a.val[m.base + 32 * k];
+      }
+    }
+    T d = 1, bi = 0, self = 0;
+    if (m.row >= 0) {
+      d = a.diag[s * 32 + lane];
+      bi = a.b[m.row];
+      self = a.old[m.row];
+    }
+    next = meta(s + nwarps);
+#pragma unroll
+    for (int k = 0; k < FLOW_WIDTH; ++k) {
+      auto& w = u[k / FLOW_GROUP][k % FLOW_GROUP];
+      w = 0;
+      if (k < m.len && !(BWD ? at[k] > m.row : at[k] < m.row)) {
+        if constexpr (sizeof(T) == 8) w = (typename S::Bits)__double_as_longlong(a.old[at[k]]);
+        else w = __float_as_uint(a.old[at[k]]);
+        at[k] = -1;  // there already
+      }
+    }
+    T sum = 0;
+#pragma unroll
+    for (int g = 0; g < FLOW_WIDTH / FLOW_GROUP; ++g) {
+#pragma unroll
+      for (int k = 0; k < FLOW_GROUP; ++k)
+        if (at[g * FLOW_GROUP + k] >= 0) u[g][k] = Fresh<T, true>::load(fresh + at[g * FLOW_GROUP + k]);
+      await<T, true>(u[g], at + g * FLOW_GROUP, fresh, m.row, a.err);
+#pragma unroll
+      for (int k = 0; k < FLOW_GROUP; ++k)
+        if (g * FLOW_GROUP + k < m.len) sum += v[g * FLOW_GROUP + k] * from_bits(u[g][k]);
+    }
+    if (m.row >= 0) {
+      const T sigma = (bi - sum) / d;
+      const typename S::Bits r = S::guard(self + a.omega * (sigma - self));
+      Fresh<T, true>::store(fresh + m.row, r);
+      a.out[m.row] = S::value(r);
+    }
+    __syncwarp();
+  }
+}
+
+template <typename T, bool BWD, bool SMEM>
+__global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a) {
+  if (a.active && *a.active != 0) return;
+  using S = Sentinel<T>;
+  constexpr unsigned ALL = 0xffffffffu;
+  extern __shared__ __align__(16) unsigned char smem[];
+  T* fresh = SMEM ? reinterpret_cast<T*>(smem) : a.out;
+  if (SMEM) {
+    for (int i = threadIdx.x; i < a.n; i += blockDim.x) fresh[i] = S::value(S::bits);
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  // Rows in order: in one CTA every nwarps-th is a warp's, else from a
+  // counter.  Either way the first row not finished reads finished rows only,
+  // and its warp is at it.
+  struct Meta {
+    int row, r0, len, d;
+  };
+  unsigned drawn = SMEM ? threadIdx.x >> 5 : lane == 0 ? atomicAdd(a.ticket, 1u) : 0u;
+  auto take = [&] {
+    const unsigned t = SMEM ? drawn : __shfl_sync(ALL, drawn, 0);
+    Meta m{-1, 0, 0, 0};
+    if (t < (unsigned)a.n) {
+      m.row = a.order[t];
+      m.r0 = a.rowptr[m.row];
+      m.len = a.rowptr[m.row + 1] - m.r0;
+      m.d = a.dpos[m.row] - m.r0;
+      if (SMEM) drawn += nwarps;
+    }
+    return m;
+  };
+  Meta next = take();
+  while (next.row >= 0) {
+    const Meta m = next;
+    if (!SMEM) drawn = lane == 0 ? atomicAdd(a.ticket, 1u) : 0u;
+    T v[FLOW_CHUNKS];
+    int at[FLOW_CHUNKS];
+    typename S::Bits u[FLOW_CHUNKS][1];
+    // a chunk's entries: coefficient, and the operand or (at >= 0) where it will be
+    auto load = [&](int q0, T& vk, int& ak, typename S::Bits& uk) {
+      const int e = q0 + lane;
+      vk = 0;
+      ak = -1;
+      uk = 0;
+      if (e >= m.len || e == m.d) return;
+      const int c = a.col[m.r0 + e];
+      vk = a.val[m.r0 + e];
+      if (BWD ? c > m.row : c < m.row) {
+        ak = c;
+        uk = S::bits;
+      } else {
+        if constexpr (sizeof(T) == 8) uk = (typename S::Bits)__double_as_longlong(a.old[c]);
+        else uk = __float_as_uint(a.old[c]);
+      }
+    };
+#pragma unroll
+    for (int c = 0; c < FLOW_CHUNKS; ++c) load(32 * c, v[c], at[c], u[c][0]);
+    const T d = a.val[m.r0 + m.d], bi = a.b[m.row], self = a.old[m.row];
+    next = take();
+    T sum = 0;
+    // a lane without an entry adds +0, which changes no sum (none is -0)
+    auto add = [&](int q0, T vk, const int& ak, typename S::Bits (&uk)[1]) {
+      await<T, SMEM>(uk, &ak, fresh, m.row, a.err);
+      const T p = vk * from_bits(uk[0]);
+      const T q = q0 + lane >= m.len || q0 + lane == m.d ? (T)0 : p;
+      const int cnt = min(32, m.len - q0);
+#pragma unroll 8
+      for (int j = 0; j < cnt; ++j) sum += __shfl_sync(ALL, q, j);
+    };
+#pragma unroll
+    for (int c = 0; c < FLOW_CHUNKS; ++c)
+      if (32 * c < m.len) add(32 * c, v[c], at[c], u[c]);
+    for (int q0 = 32 * FLOW_CHUNKS; q0 < m.len; q0 += 32) {
+      load(q0, v[0], at[0], u[0][0]);
+      add(q0, v[0], at[0], u[0]);
+    }
+    const T sigma = (bi - sum) / d;
+    const typename S::Bits r = S::guard(self + a.omega * (sigma - self));
+    if (lane == 0) {
+      Fresh<T, SMEM>::store(fresh + m.row, r);
+      if (SMEM) a.out[m.row] = S::value(r);
+    }
+    __syncwarp();
+  }
+}
+
+template <typename T>
+__global__ void k_flow_reset(int n, T* out, unsigned* ticket, const int* active) {
+  if (active && *active != 0) return;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = Sentinel<T>::value(Sentinel<T>::bits);
+  if (i == 0) *ticket = 0;
+}
+
+__global__ void k_flow_f32(int nnz, const double* __restrict__ a, float* __restrict__ b) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nnz) b[i] = (float)a[i];
+}
+
+const double* plan_val(const SweepPlan& P, double) { return P.val.get(); }
+const float* plan_val(const SweepPlan& P, float) { return P.valf.get(); }
+const double* plan_diag(const SweepPlan& P, double) { return P.diag.get(); }
+const float* plan_diag(const SweepPlan& P, float) { return P.diagf.get(); }
+
+template <typename Kernel>
+void flow_smem(std::once_flag& once, Kernel kern) {
+  std::call_once(once, [&] {
+    RSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FLOW_SMEM));
+  });
+}
+
+template <typename T, bool BWD>
+void launch_slices(Context& ctx, const char* name, const SsorArgs<T>& a) {
+  static std::once_flag once;
+  flow_smem(once, k_ssor_slices<T, BWD>);
+  RSG_LAUNCH(ctx, name, (k_ssor_slices<T, BWD>), 1, FLOW_THREADS<T>, sizeof(T) * a.n, a);
+}
+
+template <typename T, bool BWD>
+void launch_rows(Context& ctx, const char* name, const SsorArgs<T>& a) {
+  if (a.n <= FLOW_ROWS_MAX) {
+    RSG_LAUNCH(ctx, name, (k_ssor_rows<T, BWD, true>), 1, FLOW_ROW_THREADS, sizeof(T) * a.n, a);
+    return;
+  }
+  RSG_LAUNCH(ctx, name, k_flow_reset<T>, blocks_for(a.n, 256), 256, 0, a.n, a.out, a.ticket, a.active);
+  const int grid = std::min(ctx.num_sms, blocks_for((int64_t)a.n * 32, FLOW_ROW_THREADS));
+  RSG_LAUNCH(ctx, name, (k_ssor_rows<T, BWD, false>), grid, FLOW_ROW_THREADS, 0, a);
+}
+
+}  // namespace
+
+template <typename T>
+bool SsorFlow::by_slices() const {
+  return widest <= FLOW_WIDTH && sizeof(T) * (size_t)A->n <= FLOW_SMEM;
+}
+
+void SsorFlow::plan(Csr& M, const SweepPlan& fwd, const SweepPlan& bwd) {
+  ctx = M.ctx;
+  A = &M;
+  plans[0] = &fwd;
+  plans[1] = &bwd;
+  widest = 0;
+  for (int k = 0; k < M.n; ++k) widest = std::max(widest, M.h_rowptr[k + 1] - M.h_rowptr[k] - 1);
+  if (by_slices<double>()) return;  // then by_slices<float>() too
+  for (int u = 0; u < 2; ++u) {
+    const std::vector<int>& o = plans[u]->h_order;
+    order[u].resize(std::max<size_t>(o.size(), 1));
+    RSG_CUDA(cudaMemcpyAsync(order[u].get(), o.data(), sizeof(int) * o.size(), cudaMemcpyHostToDevice, ctx->stream));
+  }
+  val.resize(std::max(M.nnz, 1));
+  valf.resize(std::max(M.nnz, 1));
+  ticket.resize(1);
+}
+
+void SsorFlow::values(const double* csr) {
+  if (by_slices<double>()) return;
+  RSG_CUDA(cudaMemcpyAsync(val.get(), csr, sizeof(double) * A->nnz, cudaMemcpyDeviceToDevice, ctx->stream));
+  RSG_LAUNCH(*ctx, "flow_f32", k_flow_f32, blocks_for(A->nnz, 256), 256, 0, A->nnz, csr, valf.get());
+}
+
+template <typename T>
+void SsorFlow::sweep(bool backward, const T* b, const T* old, T* out, T omega, const int* active) {
+  const SweepPlan& P = *plans[backward ? 1 : 0];
+  const bool f32 = sizeof(T) == 4;
+  const char* name = backward ? (f32 ? "ssor_bwd_f32" : "ssor_bwd") : (f32 ? "ssor_fwd_f32" : "ssor_fwd");
+  SsorArgs<T> a{};
+  a.n = A->n;
+  a.b = b;
+  a.old = old;
+  a.out = out;
+  a.omega = omega;
+  a.active = active;
+  a.err = ctx->dev_err.get();
+  if (by_slices<T>()) {
+    a.val = plan_val(P, T());
+    a.nslices = P.nslices;
+    a.slice_base = P.slice_base.get();
+    a.row = P.row.get();
+    a.len = P.len.get();
+    a.scol = P.col.get();
+    a.diag = plan_diag(P, T());
+    if (backward) launch_slices<T, true>(*ctx, name, a);
+    else launch_slices<T, false>(*ctx, name, a);
+    return;
+  }
+  if constexpr (sizeof(T) == 8) a.val = val.get();
+  else a.val = valf.get();
+  a.order = order[backward ? 1 : 0].get();
+  a.rowptr = A->rowptr.get();
+  a.col = A->col.get();
+  a.dpos = A->diag.get();
+  a.ticket = ticket.get();
+  if (backward) launch_rows<T, true>(*ctx, name, a);
+  else launch_rows<T, false>(*ctx, name, a);
+}
+
+template void SsorFlow::sweep<double>(bool, const double*, const double*, double*, double, const int*);
+template void SsorFlow::sweep<float>(bool, const float*, const float*, float*, float, const int*);
+
+}  // namespace rsg
