@@ -202,49 +202,73 @@ __device__ void run_epilogue(int epi, KState* s, const double* t, double* hist, 
   }
 }
 
-// Block-wide deterministic sum of K values, then last-block finish.
+// Block-wide deterministic sum of K values (one or two), then last-block finish.
+//
+// A double-precision warp instruction holds its sub-partition for 64 cycles
+// whatever its active lanes, so the sums are laid out for few of them in a
+// row: the block's values go through shared memory to four warps, one per
+// sub-partition, which share the quantities, add 2 K values per lane and then
+// reduce by shuffles (700 cycles for K = 2; eight warps that shuffle both
+// quantities and a thread that adds their sums took 2300, and a block of 256
+// rows pays it for each of them; see Solver::vblk).  The state that the
+// epilogue reads is loaded before the last sums.
 template <int K>
 __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, int epi, KState* s, double* hist,
                               GmresDev g, int k) {
-  __shared__ double sh[K][RT / 32];
+  static_assert(K == 1 || K == 2, "four warps share the quantities");
+  constexpr int W = 4 / K;  // warps per quantity
+  __shared__ double sh[K][RT], sums[K][W];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int mine = w / W, at = (w % W) * 32 + lane;  // of the first four warps
 #pragma unroll
-  for (int q = 0; q < K; ++q) {
-    double x = v[q];
+  for (int q = 0; q < K; ++q) sh[q][threadIdx.x] = v[q];
+  __syncthreads();
+  auto warp_sum = [&](double x) {
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[q][w] = x;
+    if (lane == 0) sums[mine][w % W] = x;
+  };
+  auto total = [&](int q) {
+    double x = sums[q][0];
+#pragma unroll
+    for (int i = 1; i < W; ++i) x += sums[q][i];
+    return x;
+  };
+  if (w < 4) {
+    double x = sh[mine][at];
+#pragma unroll
+    for (int i = 32 * W; i < RT; i += 32 * W) x += sh[mine][at + i];
+    warp_sum(x);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < K; ++q) {
-      double x = 0;
-      for (int i = 0; i < RT / 32; ++i) x += sh[q][i];
-      part[q * gridDim.x + blockIdx.x] = x;
+  if (w == 0) {
+    if (lane < K) {
+      __stcg(part + lane * gridDim.x + blockIdx.x, total(lane));
+      __threadfence();
     }
-    __threadfence();
-    unsigned t = atomicAdd(ticket, 1u);
-    last = (t == gridDim.x - 1);
+    __syncwarp();
+    if (lane == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  double tot[K];
-#pragma unroll
-  for (int q = 0; q < K; ++q) {
+  KState c;
+  if (threadIdx.x == 0) c = *s;
+  if (w < 4) {
     double x = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += RT) x += __ldcg(part + q * gridDim.x + b);
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    __syncthreads();
-    if (lane == 0) sh[q][w] = x;
-    __syncthreads();
-    double y = 0;
-    for (int i = 0; i < RT / 32; ++i) y += sh[q][i];
-    tot[q] = y;
+#pragma unroll 4
+    for (int b = at; b < (int)gridDim.x; b += 32 * W) x += __ldcg(part + mine * gridDim.x + b);
+    warp_sum(x);
   }
+  __syncthreads();
   if (threadIdx.x == 0) {
+    double t[K];
+#pragma unroll
+    for (int q = 0; q < K; ++q) t[q] = total(q);
     *ticket = 0;
-    run_epilogue(epi, s, tot, hist, g, k);
+    run_epilogue(epi, &c, t, hist, g, k);
+    *s = c;
   }
 }
 
@@ -358,25 +382,31 @@ __global__ void __launch_bounds__(RT) k_bicg_s(int n, const double* __restrict__
   reduce_finish<1>(acc, ra.part, ra.ticket, EPI_BICG_S, ra.s, ra.hist, ra.g, 0);
 }
 
-// early exit on |s|: x.add(alpha, phat)
-__global__ void k_bicg_xfinal(int n, const double* __restrict__ phat, double* __restrict__ x, KState* s) {
-  if (*(volatile int*)&s->status != KS_CONVERGED_S) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double a = s->alpha;
-  if (i < n && a != 0) x[i] += a * phat[i];
-}
-
-__global__ void k_status_fix(KState* s) {
-  if (s->status == KS_CONVERGED_S) s->status = KS_CONVERGED;
+// The rest of an iteration that ended with |s| (status KS_CONVERGED_S): the
+// last block to get here, all having seen that status, sets the final one.
+__device__ void end_early(const RedArgs& ra) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(ra.ticket, 1u) == gridDim.x - 1) {
+    *ra.ticket = 0;
+    ra.s->status = KS_CONVERGED;
+  }
 }
 
 // x += alpha phat; x += omega shat; r = s - omega t; reduces r.r, rtilde.r
+// (x += alpha phat alone where |s| has ended the iteration)
 __global__ void __launch_bounds__(RT) k_bicg_update(int n, const double* __restrict__ phat,
                                                     const double* __restrict__ shat, const double* __restrict__ sv,
                                                     const double* __restrict__ t, const double* __restrict__ rtilde,
                                                     double* __restrict__ x, double* __restrict__ r, RedArgs ra) {
-  if (stopped(ra.s)) return;
+  const int status = *(volatile const int*)&ra.s->status;
+  if (status != 0 && status != KS_CONVERGED_S) return;
   const double alpha = ra.s->alpha, omega = ra.s->omega, mo = -omega;
+  if (status == KS_CONVERGED_S) {  // x.add(alpha, phat)
+    for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT)
+      if (alpha != 0) x[i] += alpha * phat[i];
+    end_early(ra);
+    return;
+  }
   double acc[2] = {0, 0};
   for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT) {
     double xi = x[i];
@@ -563,18 +593,18 @@ __global__ void __launch_bounds__(RT) k_f32_bicg_s(int n, const float* __restric
   reduce_finish<1>(acc, ra.part, ra.ticket, EPI_BICG_S_IN, ra.s, ra.hist, ra.g, 0);
 }
 
-__global__ void k_f32_bicg_xfinal(int n, const float* __restrict__ phat, float* __restrict__ x, KState* s) {
-  if (*(volatile int*)&s->status != KS_CONVERGED_S) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] += (float)s->alpha * phat[i];
-}
-
 __global__ void __launch_bounds__(RT) k_f32_bicg_update(int n, const float* __restrict__ phat,
                                                         const float* __restrict__ shat, const float* __restrict__ sv,
                                                         const float* __restrict__ t, const float* __restrict__ rtilde,
                                                         float* __restrict__ x, float* __restrict__ r, RedArgs ra) {
-  if (stopped(ra.s)) return;
+  const int status = *(volatile const int*)&ra.s->status;
+  if (status != 0 && status != KS_CONVERGED_S) return;
   const float alpha = (float)ra.s->alpha, omega = (float)ra.s->omega;
+  if (status == KS_CONVERGED_S) {
+    for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT) x[i] += alpha * phat[i];
+    end_early(ra);
+    return;
+  }
   double acc[2] = {0, 0};
   for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT) {
     x[i] = x[i] + alpha * phat[i] + omega * shat[i];
@@ -615,7 +645,10 @@ struct Solver {
   DeviceBuffer<unsigned> ticket_in;
   DeviceBuffer<KState> state_in;
   KState* hstate = nullptr;  // pinned mirror
-  int nblk = 0;
+  // Blocks of the kernels with reductions: SpMV (eight resident per SM) and
+  // vectors.  More would be further rounds of the block's sums: 16 of the 30 us
+  // of an update of 524,288 rows went there with a block per 256 rows.
+  int nblk = 0, vblk = 0;
   Csr* setup_for = nullptr;
 
   Solver(Context* c, int m, int p) : ctx(c), method(m), pc_kind(p) {
@@ -639,7 +672,8 @@ struct Solver {
       b->resize(n);
       RSG_CUDA(cudaMemsetAsync(b->get(), 0, sizeof(double) * n, ctx->stream));
     }
-    nblk = std::max(1, std::min(blocks_for(n, RT), 16384));
+    nblk = std::max(1, std::min(blocks_for(n, RT), 8 * ctx->num_sms));
+    vblk = std::max(1, std::min(blocks_for(n, RT), 4 * ctx->num_sms));
     part.resize((size_t)4 * nblk);
   }
 
@@ -721,13 +755,11 @@ struct Solver {
         pc->apply(p, ph, act);
         RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), ph, v, rt, red(), (int)EPI_BICG_ALPHA);
-        RSG_LAUNCH(*ctx, "bicg_s", k_bicg_s, nblk, RT, 0, n, r, v, s, red());
-        RSG_LAUNCH(*ctx, "bicg_xfinal", k_bicg_xfinal, eb, 256, 0, n, ph, x, state.get());
-        RSG_LAUNCH(*ctx, "status_fix", k_status_fix, 1, 1, 0, state.get());
+        RSG_LAUNCH(*ctx, "bicg_s", k_bicg_s, vblk, RT, 0, n, r, v, s, red());
         pc->apply(s, sh, act);
         RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), sh, t, s, red(), (int)EPI_BICG_OMEGA);
-        RSG_LAUNCH(*ctx, "bicg_update", k_bicg_update, nblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
+        RSG_LAUNCH(*ctx, "bicg_update", k_bicg_update, vblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
       }
     }
   }
@@ -743,11 +775,11 @@ struct Solver {
       if (hstate->status != 0) break;
       for (int it = 0; it < batch(); ++it) {
         pc->apply(r, z, act);
-        RSG_LAUNCH(*ctx, "dot", k_dot, nblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
+        RSG_LAUNCH(*ctx, "dot", k_dot, vblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
         RSG_LAUNCH(*ctx, "cg_p", k_cg_p, eb, 256, 0, n, z, p, state.get());
         RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), p, q, p, red(), (int)EPI_CG_ALPHA);
-        RSG_LAUNCH(*ctx, "cg_update", k_cg_update, nblk, RT, 0, n, p, q, x, r, red());
+        RSG_LAUNCH(*ctx, "cg_update", k_cg_update, vblk, RT, 0, n, p, q, x, r, red());
       }
     }
   }
@@ -789,7 +821,7 @@ struct Solver {
     // r = b - A x; monitor(|r|)
     RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
-    RSG_LAUNCH(*ctx, "fgm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    RSG_LAUNCH(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     for (;;) {
       read_state();
       if (hstate->status != 0) break;
@@ -798,27 +830,25 @@ struct Solver {
         const int i = hstate->gm_i;
         // z_i = M(v_i): FP32 BiCGstab + ILU(0) from zero
         RSG_LAUNCH(*ctx, "inner_reset", k_inner_reset, 1, 1, 0, sin, inner_rtol, 0.0, inner_iters);
-        RSG_LAUNCH(*ctx, "inner_init", k_f32_init, nblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
+        RSG_LAUNCH(*ctx, "inner_init", k_f32_init, vblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
         for (int q = 0; q < inner_iters; ++q) {
           RSG_LAUNCH(*ctx, "inner_p", k_f32_bicg_p, eb, 256, 0, n, ir, iv, ip, sin);
           pc->apply_f32(ip, iph, act_in);
           RSG_LAUNCH(*ctx, "inner_spmv_dot", k_f32_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), iph, iv, irt, ri, (int)EPI_BICG_ALPHA);
-          RSG_LAUNCH(*ctx, "inner_s", k_f32_bicg_s, nblk, RT, 0, n, ir, iv, is, ri);
-          RSG_LAUNCH(*ctx, "inner_xfinal", k_f32_bicg_xfinal, eb, 256, 0, n, iph, ix, sin);
-          RSG_LAUNCH(*ctx, "status_fix", k_status_fix, 1, 1, 0, sin);
+          RSG_LAUNCH(*ctx, "inner_s", k_f32_bicg_s, vblk, RT, 0, n, ir, iv, is, ri);
           pc->apply_f32(is, ish, act_in);
           RSG_LAUNCH(*ctx, "inner_spmv_dot", k_f32_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), ish, it, is, ri, (int)EPI_BICG_OMEGA);
-          RSG_LAUNCH(*ctx, "inner_update", k_f32_bicg_update, nblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
+          RSG_LAUNCH(*ctx, "inner_update", k_f32_bicg_update, vblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
         }
         RSG_LAUNCH(*ctx, "to_f64", k_f32_to_f64, eb, 256, 0, n, ix, zcol(i), (const KState*)sin, state.get());
         // w = A z_i, then the Arnoldi step of GMRES.java:146-162 on w
         launch_spmv(*ctx, A, zcol(i), w, nullptr);
         for (int k2 = 0; k2 <= i; ++k2)
-          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
+          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
                      vcol(k2), red(), k2, (int)EPI_GM_H);
-        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
         RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
@@ -829,7 +859,7 @@ struct Solver {
       RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                  A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      RSG_LAUNCH(*ctx, "fgm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      RSG_LAUNCH(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 
@@ -849,7 +879,7 @@ struct Solver {
     RSG_LAUNCH(*ctx, "gm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
     pc->apply(u, r, nullptr);
-    RSG_LAUNCH(*ctx, "gm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    RSG_LAUNCH(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     pc->apply(b, u, nullptr);
     for (;;) {
       read_state();
@@ -861,9 +891,9 @@ struct Solver {
         launch_spmv(*ctx, A, vcol(i), u, nullptr);
         pc->apply(u, w, nullptr);
         for (int k = 0; k <= i; ++k)
-          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
+          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
                      vcol(k), red(), k, (int)EPI_GM_H);
-        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
         RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
@@ -876,7 +906,7 @@ struct Solver {
                  A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
       pc->apply(u, r, nullptr);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      RSG_LAUNCH(*ctx, "gm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      RSG_LAUNCH(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 };
