@@ -631,6 +631,7 @@ struct BlockWalkIo {
 
 template <typename T, bool UPPER, int D>
 __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, BlockWalkIo<T> io) {
+  chain_begin();
   if (io.active && *io.active != 0) return;
   using S = Sentinel<T>;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -860,7 +861,7 @@ void launch(Context& ctx, const char* name, const BlockWalk& P, const BlockWalkI
   });
   const BlockWalkArgs g{P.blk_step.get(), P.hptr.get(), P.hsrc.get(), P.ints.get(), P.bsrc.get(), P.w, P.nblk, P.halo,
                         (int)P.own_old, P.ticket.get(), ctx.dev_err.get()};
-  RSG_LAUNCH(ctx, name, kern, P.nblk, BW_THREADS, smem, g, io);
+  launch_chained(ctx, name, kern, P.nblk, BW_THREADS, smem, g, io);
 }
 
 }  // namespace

@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(RT, 8) k_spmv_dot(int n, const int* __restrict
                                                  const int* __restrict__ col, const double* __restrict__ val,
                                                  const double* __restrict__ x, double* __restrict__ y,
                                                  const double* __restrict__ w, RedArgs ra, int epi) {
+  chain_begin();
   if (stopped(ra.s)) return;
   double v[K];
 #pragma unroll
@@ -344,6 +345,7 @@ __global__ void __launch_bounds__(RT, 8) k_spmv_dot(int n, const int* __restrict
 // Generic dot a.b
 __global__ void __launch_bounds__(RT) k_dot(int n, const double* __restrict__ a, const double* __restrict__ b,
                                             RedArgs ra, int epi, int k) {
+  chain_begin();
   if (stopped(ra.s)) return;
   double v[1] = {0};
   for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT) v[0] += a[i] * b[i];
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(RT) k_dot(int n, const double* __restrict__ a,
 // ---- BiCGstab elementwise steps
 __global__ void k_bicg_p(int n, const double* __restrict__ r, const double* __restrict__ v, double* __restrict__ p,
                          const KState* s) {
+  chain_begin();
   if (stopped(s)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -371,6 +374,7 @@ __global__ void k_bicg_p(int n, const double* __restrict__ r, const double* __re
 // s = r - alpha v (s.set(r).add(-alpha, v)), reduces s.s
 __global__ void __launch_bounds__(RT) k_bicg_s(int n, const double* __restrict__ r, const double* __restrict__ v,
                                                double* __restrict__ sv, RedArgs ra) {
+  chain_begin();
   if (stopped(ra.s)) return;
   const double ma = -ra.s->alpha;
   double acc[1] = {0};
@@ -398,6 +402,7 @@ __global__ void __launch_bounds__(RT) k_bicg_update(int n, const double* __restr
                                                     const double* __restrict__ shat, const double* __restrict__ sv,
                                                     const double* __restrict__ t, const double* __restrict__ rtilde,
                                                     double* __restrict__ x, double* __restrict__ r, RedArgs ra) {
+  chain_begin();
   const int status = *(volatile const int*)&ra.s->status;
   if (status != 0 && status != KS_CONVERGED_S) return;
   const double alpha = ra.s->alpha, omega = ra.s->omega, mo = -omega;
@@ -423,6 +428,7 @@ __global__ void __launch_bounds__(RT) k_bicg_update(int n, const double* __restr
 
 // ---- CG elementwise steps
 __global__ void k_cg_p(int n, const double* __restrict__ z, double* __restrict__ p, const KState* s) {
+  chain_begin();
   if (stopped(s)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -436,6 +442,7 @@ __global__ void k_cg_p(int n, const double* __restrict__ z, double* __restrict__
 // x += alpha p; r += -alpha q; reduces r.r
 __global__ void __launch_bounds__(RT) k_cg_update(int n, const double* __restrict__ p, const double* __restrict__ q,
                                                   double* __restrict__ x, double* __restrict__ r, RedArgs ra) {
+  chain_begin();
   if (stopped(ra.s)) return;
   const double alpha = ra.s->alpha, ma = -alpha;
   double acc[1] = {0};
@@ -453,6 +460,7 @@ __global__ void __launch_bounds__(RT) k_cg_update(int n, const double* __restric
 // w += -H(k-1,i) v_{k-1} (when k > 0), then reduce w.v_k (k <= i) or w.w (k = i+1)
 __global__ void __launch_bounds__(RT) k_gm_mgs(int n, double* __restrict__ w, const double* __restrict__ vprev,
                                                const double* __restrict__ vk, RedArgs ra, int k, int epi) {
+  chain_begin();
   if (stopped(ra.s)) return;
   const int i = ra.s->gm_i, ld = ra.s->restart + 1;
   const double h = (k > 0) ? -ra.g.H[(k - 1) + i * ld] : 0.0;
@@ -470,6 +478,7 @@ __global__ void __launch_bounds__(RT) k_gm_mgs(int n, double* __restrict__ w, co
 
 // y.set(alpha, x) with alpha = KState.vscale
 __global__ void k_gm_vset(int n, const double* __restrict__ w, double* __restrict__ v, const KState* s) {
+  chain_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double a = s->vscale;
@@ -512,6 +521,7 @@ __global__ void k_iter_inc(KState* s) { s->iter++; }
 // preconditioner are FP32; dot products accumulate in FP64 and the scalar
 // recurrences (KState) stay FP64.
 __global__ void k_inner_reset(KState* s, double rtol, double atol, int maxIter) {
+  chain_begin();
   KState z = {};
   z.rho_1 = z.rho_2 = z.alpha = z.beta = z.omega = 1;
   z.rtol = rtol;
@@ -526,6 +536,7 @@ __global__ void k_inner_reset(KState* s, double rtol, double atol, int maxIter) 
 // r = rt = (float) v (x0 = 0), x = 0; reduces r.r twice (rtilde.r = r.r)
 __global__ void __launch_bounds__(RT) k_f32_init(int n, const double* __restrict__ v, float* __restrict__ r,
                                                  float* __restrict__ rt, float* __restrict__ x, RedArgs ra) {
+  chain_begin();
   double acc[2] = {0, 0};
   for (int i = blockIdx.x * RT + threadIdx.x; i < n; i += gridDim.x * RT) {
     float ri = (float)v[i];
@@ -540,6 +551,7 @@ __global__ void __launch_bounds__(RT) k_f32_init(int n, const double* __restrict
 
 __global__ void k_f32_bicg_p(int n, const float* __restrict__ r, const float* __restrict__ v, float* __restrict__ p,
                              const KState* s) {
+  chain_begin();
   if (stopped(s)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -557,6 +569,7 @@ __global__ void __launch_bounds__(RT, 8) k_f32_spmv_dot(int n, const int* __rest
                                                      const int* __restrict__ col, const float* __restrict__ val,
                                                      const float* __restrict__ x, float* __restrict__ y,
                                                      const float* __restrict__ w, RedArgs ra, int epi) {
+  chain_begin();
   if (stopped(ra.s)) return;
   double v[K];
 #pragma unroll
@@ -582,6 +595,7 @@ __global__ void __launch_bounds__(RT, 8) k_f32_spmv_dot(int n, const int* __rest
 
 __global__ void __launch_bounds__(RT) k_f32_bicg_s(int n, const float* __restrict__ r, const float* __restrict__ v,
                                                    float* __restrict__ sv, RedArgs ra) {
+  chain_begin();
   if (stopped(ra.s)) return;
   const float ma = (float)(-ra.s->alpha);
   double acc[1] = {0};
@@ -597,6 +611,7 @@ __global__ void __launch_bounds__(RT) k_f32_bicg_update(int n, const float* __re
                                                         const float* __restrict__ shat, const float* __restrict__ sv,
                                                         const float* __restrict__ t, const float* __restrict__ rtilde,
                                                         float* __restrict__ x, float* __restrict__ r, RedArgs ra) {
+  chain_begin();
   const int status = *(volatile const int*)&ra.s->status;
   if (status != 0 && status != KS_CONVERGED_S) return;
   const float alpha = (float)ra.s->alpha, omega = (float)ra.s->omega;
@@ -618,6 +633,7 @@ __global__ void __launch_bounds__(RT) k_f32_bicg_update(int n, const float* __re
 
 __global__ void k_f32_to_f64(int n, const float* __restrict__ a, double* __restrict__ b, const KState* sin,
                              KState* sout) {
+  chain_begin();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (double)a[i];
   if (i == 0) sout->inner += sin->iter;
@@ -751,15 +767,15 @@ struct Solver {
       read_state();
       if (hstate->status != 0) break;
       for (int it = 0; it < batch(); ++it) {
-        RSG_LAUNCH(*ctx, "bicg_p", k_bicg_p, eb, 256, 0, n, r, v, p, state.get());
+        launch_chained(*ctx, "bicg_p", k_bicg_p, eb, 256, 0, n, r, v, p, state.get());
         pc->apply(p, ph, act);
-        RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
+        launch_chained(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), ph, v, rt, red(), (int)EPI_BICG_ALPHA);
-        RSG_LAUNCH(*ctx, "bicg_s", k_bicg_s, vblk, RT, 0, n, r, v, s, red());
+        launch_chained(*ctx, "bicg_s", k_bicg_s, vblk, RT, 0, n, r, v, s, red());
         pc->apply(s, sh, act);
-        RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
+        launch_chained(*ctx, "spmv_dot", k_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), sh, t, s, red(), (int)EPI_BICG_OMEGA);
-        RSG_LAUNCH(*ctx, "bicg_update", k_bicg_update, vblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
+        launch_chained(*ctx, "bicg_update", k_bicg_update, vblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
       }
     }
   }
@@ -775,11 +791,11 @@ struct Solver {
       if (hstate->status != 0) break;
       for (int it = 0; it < batch(); ++it) {
         pc->apply(r, z, act);
-        RSG_LAUNCH(*ctx, "dot", k_dot, vblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
-        RSG_LAUNCH(*ctx, "cg_p", k_cg_p, eb, 256, 0, n, z, p, state.get());
-        RSG_LAUNCH(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
+        launch_chained(*ctx, "dot", k_dot, vblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
+        launch_chained(*ctx, "cg_p", k_cg_p, eb, 256, 0, n, z, p, state.get());
+        launch_chained(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), p, q, p, red(), (int)EPI_CG_ALPHA);
-        RSG_LAUNCH(*ctx, "cg_update", k_cg_update, vblk, RT, 0, n, p, q, x, r, red());
+        launch_chained(*ctx, "cg_update", k_cg_update, vblk, RT, 0, n, p, q, x, r, red());
       }
     }
   }
@@ -821,36 +837,36 @@ struct Solver {
     // r = b - A x; monitor(|r|)
     RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
-    RSG_LAUNCH(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    launch_chained(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     for (;;) {
       read_state();
       if (hstate->status != 0) break;
-      RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, r, vcol(0), state.get());
+      launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, r, vcol(0), state.get());
       while (!hstate->gm_exit && hstate->status == 0) {
         const int i = hstate->gm_i;
         // z_i = M(v_i): FP32 BiCGstab + ILU(0) from zero
-        RSG_LAUNCH(*ctx, "inner_reset", k_inner_reset, 1, 1, 0, sin, inner_rtol, 0.0, inner_iters);
-        RSG_LAUNCH(*ctx, "inner_init", k_f32_init, vblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
+        launch_chained(*ctx, "inner_reset", k_inner_reset, 1, 1, 0, sin, inner_rtol, 0.0, inner_iters);
+        launch_chained(*ctx, "inner_init", k_f32_init, vblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
         for (int q = 0; q < inner_iters; ++q) {
-          RSG_LAUNCH(*ctx, "inner_p", k_f32_bicg_p, eb, 256, 0, n, ir, iv, ip, sin);
+          launch_chained(*ctx, "inner_p", k_f32_bicg_p, eb, 256, 0, n, ir, iv, ip, sin);
           pc->apply_f32(ip, iph, act_in);
-          RSG_LAUNCH(*ctx, "inner_spmv_dot", k_f32_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
+          launch_chained(*ctx, "inner_spmv_dot", k_f32_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), iph, iv, irt, ri, (int)EPI_BICG_ALPHA);
-          RSG_LAUNCH(*ctx, "inner_s", k_f32_bicg_s, vblk, RT, 0, n, ir, iv, is, ri);
+          launch_chained(*ctx, "inner_s", k_f32_bicg_s, vblk, RT, 0, n, ir, iv, is, ri);
           pc->apply_f32(is, ish, act_in);
-          RSG_LAUNCH(*ctx, "inner_spmv_dot", k_f32_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
+          launch_chained(*ctx, "inner_spmv_dot", k_f32_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), ish, it, is, ri, (int)EPI_BICG_OMEGA);
-          RSG_LAUNCH(*ctx, "inner_update", k_f32_bicg_update, vblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
+          launch_chained(*ctx, "inner_update", k_f32_bicg_update, vblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
         }
-        RSG_LAUNCH(*ctx, "to_f64", k_f32_to_f64, eb, 256, 0, n, ix, zcol(i), (const KState*)sin, state.get());
+        launch_chained(*ctx, "to_f64", k_f32_to_f64, eb, 256, 0, n, ix, zcol(i), (const KState*)sin, state.get());
         // w = A z_i, then the Arnoldi step of GMRES.java:146-162 on w
         launch_spmv(*ctx, A, zcol(i), w, nullptr);
         for (int k2 = 0; k2 <= i; ++k2)
-          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
+          launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
                      vcol(k2), red(), k2, (int)EPI_GM_H);
-        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
-        RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
+        launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
       }
       if (hstate->status != 0) break;
@@ -859,7 +875,7 @@ struct Solver {
       RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                  A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      RSG_LAUNCH(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      launch_chained(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 
@@ -879,23 +895,23 @@ struct Solver {
     RSG_LAUNCH(*ctx, "gm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
     pc->apply(u, r, nullptr);
-    RSG_LAUNCH(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    launch_chained(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     pc->apply(b, u, nullptr);
     for (;;) {
       read_state();
       if (hstate->status != 0) break;
       // v[0] = r / normr
-      RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, r, vcol(0), state.get());
+      launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, r, vcol(0), state.get());
       while (!hstate->gm_exit && hstate->status == 0) {
         const int i = hstate->gm_i;
         launch_spmv(*ctx, A, vcol(i), u, nullptr);
         pc->apply(u, w, nullptr);
         for (int k = 0; k <= i; ++k)
-          RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
+          launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
                      vcol(k), red(), k, (int)EPI_GM_H);
-        RSG_LAUNCH(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
-        RSG_LAUNCH(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
+        launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
       }
       if (hstate->status != 0) break;
@@ -906,7 +922,7 @@ struct Solver {
                  A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
       pc->apply(u, r, nullptr);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      RSG_LAUNCH(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      launch_chained(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 };
