@@ -12,12 +12,17 @@
 //    A warp's slices are far apart in the order, so the loads of one pass
 //    behind the chain of the slices before it.
 //  * Wider rows (Galerkin products): a warp per row, a lane per entry, the
-//    lanes' products summed in order through shuffles.  One CTA while the
-//    rows are few; all SMs, with the values polled through L2, for more.
-// The V-cycle sweeps of a 40 x 36 x 12 system in FP32: 27 us on the 17,280
-// rows (slices) and 34 us on average on the three coarse levels (a warp per
-// row), against 245 us on average on one 8-CTA cluster with a barrier per
-// level.  That solve with its setup: 71 ms against 285.
+//    lanes' products summed in order through shuffles (FP64).  One CTA while
+//    the rows are few; all SMs, with the values polled through L2, for more.
+// FP32 sweeps are the mixed-precision solver's own and owe no order to the Java
+// loop.  There a warp's row leaves the operand that comes last (of the highest
+// level) out of the sum, adds the others by a tree while it waits for it, and
+// has one multiply-add left when it is there.
+// The V-cycle sweeps of a 40 x 36 x 12 system in FP32: 26 us on the 17,280
+// rows (slices) and 20 us on average on the three coarse levels (a warp per
+// row; 34 us with the ordered sum), against 245 us on average on one 8-CTA
+// cluster with a barrier per level.  That solve with its setup: 58 ms (72 with
+// the ordered sums) against 285.
 #include <mutex>
 
 #include "dataflow.cuh"
@@ -87,6 +92,7 @@ struct SsorArgs {
   const T* diag;
   // rows
   const int *order, *rowptr, *col, *dpos;
+  const int* newest;  // entry of the row that is computed last, -1 none
   unsigned* ticket;
 };
 
@@ -193,6 +199,7 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
   if (a.active && *a.active != 0) return;
   using S = Sentinel<T>;
   constexpr unsigned ALL = 0xffffffffu;
+  constexpr bool TREE = sizeof(T) == 4;
   extern __shared__ __align__(16) unsigned char smem[];
   T* fresh = SMEM ? reinterpret_cast<T*>(smem) : a.out;
   if (SMEM) {
@@ -204,17 +211,18 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
   // counter.  Either way the first row not finished reads finished rows only,
   // and its warp is at it.
   struct Meta {
-    int row, r0, len, d;
+    int row, r0, len, d, newest;
   };
   unsigned drawn = SMEM ? threadIdx.x >> 5 : lane == 0 ? atomicAdd(a.ticket, 1u) : 0u;
   auto take = [&] {
     const unsigned t = SMEM ? drawn : __shfl_sync(ALL, drawn, 0);
-    Meta m{-1, 0, 0, 0};
+    Meta m{-1, 0, 0, 0, -1};
     if (t < (unsigned)a.n) {
       m.row = a.order[t];
       m.r0 = a.rowptr[m.row];
       m.len = a.rowptr[m.row + 1] - m.r0;
       m.d = a.dpos[m.row] - m.r0;
+      if (TREE) m.newest = a.newest[m.row];
       if (SMEM) drawn += nwarps;
     }
     return m;
@@ -232,7 +240,7 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
       vk = 0;
       ak = -1;
       uk = 0;
-      if (e >= m.len || e == m.d) return;
+      if (e >= m.len || e == m.d || e == m.newest) return;
       const int c = a.col[m.r0 + e];
       vk = a.val[m.r0 + e];
       if (BWD ? c > m.row : c < m.row) {
@@ -248,6 +256,34 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
     const T d = a.val[m.r0 + m.d], bi = a.b[m.row], self = a.old[m.row];
     next = take();
     T sum = 0;
+    if constexpr (TREE) {
+      const int nq = m.r0 + max(m.newest, 0);
+      const T nv = m.newest >= 0 ? a.val[nq] : (T)0;
+      const int nc = m.newest >= 0 ? a.col[nq] : -1;
+      const T w = a.omega / d;
+#pragma unroll
+      for (int c = 0; c < FLOW_CHUNKS; ++c) {
+        await<T, SMEM>(u[c], &at[c], fresh, m.row, a.err);
+        sum = fmaf(v[c], from_bits(u[c][0]), sum);
+      }
+      for (int q0 = 32 * FLOW_CHUNKS; q0 < m.len; q0 += 32) {
+        load(q0, v[0], at[0], u[0][0]);
+        await<T, SMEM>(u[0], &at[0], fresh, m.row, a.err);
+        sum = fmaf(v[0], from_bits(u[0][0]), sum);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(ALL, sum, o);
+      const T rest = fmaf(w, bi - sum, self - a.omega * self);
+      typename S::Bits last[1] = {nc >= 0 ? S::bits : 0};
+      await<T, SMEM>(last, &nc, fresh, m.row, a.err);
+      const typename S::Bits r = S::guard(fmaf(-(w * nv), from_bits(last[0]), rest));
+      if (lane == 0) {
+        Fresh<T, SMEM>::store(fresh + m.row, r);
+        if (SMEM) a.out[m.row] = S::value(r);
+      }
+      __syncwarp();
+      continue;
+    }
     // a lane without an entry adds +0, which changes no sum (none is -0)
     auto add = [&](int q0, T vk, const int& ak, typename S::Bits (&uk)[1]) {
       await<T, SMEM>(uk, &ak, fresh, m.row, a.err);
@@ -335,6 +371,23 @@ void SsorFlow::plan(Csr& M, const SweepPlan& fwd, const SweepPlan& bwd) {
   for (int u = 0; u < 2; ++u) {
     const std::vector<int>& o = plans[u]->h_order;
     order[u].resize(std::max<size_t>(o.size(), 1));
+    // the entry of the highest level of each row, of several the one nearest
+    // the diagonal (on a grid it is computed last)
+    std::vector<int> lev(M.n, 0), entry(std::max(M.n, 1), -1);
+    for (int row : o) {
+      const int r0 = M.h_rowptr[row], d = M.h_diag[row], r1 = M.h_rowptr[row + 1];
+      int top = -1;
+      for (int q = u ? r1 - 1 : r0; u ? q > d : q < d; u ? --q : ++q)
+        if (lev[M.h_col[q]] >= top) {
+          top = lev[M.h_col[q]];
+          entry[row] = q - r0;
+        }
+      lev[row] = top + 1;
+    }
+    newest[u].resize(entry.size());
+    RSG_CUDA(cudaMemcpyAsync(newest[u].get(), entry.data(), sizeof(int) * entry.size(), cudaMemcpyHostToDevice,
+                             ctx->stream));
+    ctx->sync();  // entry goes out of scope
     RSG_CUDA(cudaMemcpyAsync(order[u].get(), o.data(), sizeof(int) * o.size(), cudaMemcpyHostToDevice, ctx->stream));
   }
   val.resize(std::max(M.nnz, 1));
@@ -376,6 +429,7 @@ void SsorFlow::sweep(bool backward, const T* b, const T* old, T* out, T omega, c
   if constexpr (sizeof(T) == 8) a.val = val.get();
   else a.val = valf.get();
   a.order = order[backward ? 1 : 0].get();
+  a.newest = newest[backward ? 1 : 0].get();
   a.rowptr = A->rowptr.get();
   a.col = A->col.get();
   a.dpos = A->diag.get();

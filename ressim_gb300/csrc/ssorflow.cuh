@@ -22,7 +22,7 @@ struct SsorFlow {
   Csr* A = nullptr;
   const SweepPlan* plans[2] = {nullptr, nullptr};
   int widest = 0;  // longest row, without its diagonal
-  DeviceBuffer<int> order[2];
+  DeviceBuffer<int> order[2], newest[2];
   DeviceBuffer<double> val;  // by CSR position, where the rows kernel runs
   DeviceBuffer<float> valf;
   DeviceBuffer<unsigned> ticket;
