@@ -561,6 +561,7 @@ __global__ void k_dense_lu(int n, const int* __restrict__ rp, const int* __restr
 // directSolve (AMG.java:315-323): u = f, then dgetrs ('N' or 'T')
 __global__ void k_dense_solve(int n, const double* __restrict__ A, const int* __restrict__ piv,
                               const double* __restrict__ f, double* __restrict__ u, int trans, const int* active) {
+  chain_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (active && *active != 0) return;
   for (int i = 0; i < n; ++i) u[i] = f[i];
@@ -607,6 +608,7 @@ template <typename T>
 __global__ void k_amg_resid(int n, const int* __restrict__ rp, const int* __restrict__ col,
                             const T* __restrict__ val, const T* __restrict__ u, const T* __restrict__ f,
                             T* __restrict__ r, const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -620,6 +622,7 @@ template <typename T>
 __global__ void k_amg_restrict(int c, const int* __restrict__ qptr, const int* __restrict__ qrow,
                                const T* __restrict__ qval, const T* __restrict__ r, T* __restrict__ f,
                                const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= c) return;
@@ -634,6 +637,7 @@ template <typename T>
 __global__ void k_amg_prolong(int n, const int* __restrict__ prp, const int* __restrict__ pcol,
                               const T* __restrict__ pval, const T* __restrict__ un, T* __restrict__ u,
                               const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -644,6 +648,7 @@ __global__ void k_amg_prolong(int n, const int* __restrict__ prp, const int* __r
 
 template <typename A, typename B>
 __global__ void k_amg_copy(int n, const A* __restrict__ a, B* __restrict__ b, const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = (B)a[i];
@@ -651,6 +656,7 @@ __global__ void k_amg_copy(int n, const A* __restrict__ a, B* __restrict__ b, co
 
 template <typename T>
 __global__ void k_amg_zero(int n, T* __restrict__ b, const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = 0;
@@ -865,7 +871,7 @@ struct AMGPrecond : Precond {
     const int n = l.A->n;
     if (k == m - 1) {
       if (info > 0) throw Error(RSG_SINGULAR, "MatrixSingularException: the coarsest AMG operator is singular");
-      RSG_LAUNCH(c, "amg_direct", k_dense_solve, 1, 32, 0, nc, lu.get(), piv.get(), l.f.get(), l.u.get(),
+      launch_chained(c, "amg_direct", k_dense_solve, 1, 32, 0, nc, lu.get(), piv.get(), l.f.get(), l.u.get(),
                  trans ? 1 : 0, active);
       return;
     }
@@ -873,13 +879,13 @@ struct AMGPrecond : Precond {
     const int eb = blocks_for(n, 256);
     set_ssor_params(l.smoother.get(), 1.0, 1.85, 1);  // preRelax: SSOR(omegaPreF, omegaPreR)
     l.smoother->apply(l.f.get(), l.u.get(), active);
-    RSG_LAUNCH(c, "amg_zero", k_amg_zero<double>, blocks_for(nx.A->n, 256), 256, 0, nx.A->n, nx.u.get(), active);
-    RSG_LAUNCH(c, "amg_resid", k_amg_resid<double>, eb, 256, 0, n, l.A->rowptr.get(), l.A->col.get(), l.val,
+    launch_chained(c, "amg_zero", k_amg_zero<double>, blocks_for(nx.A->n, 256), 256, 0, nx.A->n, nx.u.get(), active);
+    launch_chained(c, "amg_resid", k_amg_resid<double>, eb, 256, 0, n, l.A->rowptr.get(), l.A->col.get(), l.val,
                l.u.get(), l.f.get(), l.r.get(), active);
-    RSG_LAUNCH(c, "amg_restrict", k_amg_restrict<double>, blocks_for(l.c, 256), 256, 0, l.c, l.qptr.get(),
+    launch_chained(c, "amg_restrict", k_amg_restrict<double>, blocks_for(l.c, 256), 256, 0, l.c, l.qptr.get(),
                l.qrow.get(), l.qval.get(), l.r.get(), nx.f.get(), active);
     cycle(k + 1, active);
-    RSG_LAUNCH(c, "amg_prolong", k_amg_prolong<double>, eb, 256, 0, n, l.prp.get(), l.pcol.get(), l.pval.get(),
+    launch_chained(c, "amg_prolong", k_amg_prolong<double>, eb, 256, 0, n, l.prp.get(), l.pcol.get(), l.pval.get(),
                nx.u.get(), l.u.get(), active);
     set_ssor_params(l.smoother.get(), 1.85, 1.0, 1);  // postRelax: SSOR(omegaPostF, omegaPostR)
     l.smoother->apply(l.f.get(), l.u.get(), active);
@@ -890,11 +896,11 @@ struct AMGPrecond : Precond {
     Context& c = *ctx;
     const int n = L[0].A->n;
     const int eb = blocks_for(n, 256);
-    RSG_LAUNCH(c, "amg_copy", (k_amg_copy<double, double>), eb, 256, 0, n, x, L[0].u.get(), active);
-    RSG_LAUNCH(c, "amg_copy", (k_amg_copy<double, double>), eb, 256, 0, n, b, L[0].f.get(), active);
+    launch_chained(c, "amg_copy", k_amg_copy<double, double>, eb, 256, 0, n, x, L[0].u.get(), active);
+    launch_chained(c, "amg_copy", k_amg_copy<double, double>, eb, 256, 0, n, b, L[0].f.get(), active);
     trans = t;
     cycle(0, active);
-    RSG_LAUNCH(c, "amg_copy", (k_amg_copy<double, double>), eb, 256, 0, n, L[0].u.get(), x, active);
+    launch_chained(c, "amg_copy", k_amg_copy<double, double>, eb, 256, 0, n, L[0].u.get(), x, active);
   }
 
   // FP32 copy of the hierarchy, made on the first FP32 apply after a setup:
@@ -931,21 +937,21 @@ struct AMGPrecond : Precond {
     const int eb = blocks_for(n, 256);
     if (k == m - 1) {
       if (info > 0) throw Error(RSG_SINGULAR, "MatrixSingularException: the coarsest AMG operator is singular");
-      RSG_LAUNCH(c, "amg_coarse_cvt", (k_amg_copy<float, double>), eb, 256, 0, n, l.ff.get(), l.f.get(), active);
-      RSG_LAUNCH(c, "amg_direct", k_dense_solve, 1, 32, 0, nc, lu.get(), piv.get(), l.f.get(), l.u.get(), 0, active);
-      RSG_LAUNCH(c, "amg_coarse_cvt", (k_amg_copy<double, float>), eb, 256, 0, n, l.u.get(), l.uf.get(), active);
+      launch_chained(c, "amg_coarse_cvt", k_amg_copy<float, double>, eb, 256, 0, n, l.ff.get(), l.f.get(), active);
+      launch_chained(c, "amg_direct", k_dense_solve, 1, 32, 0, nc, lu.get(), piv.get(), l.f.get(), l.u.get(), 0, active);
+      launch_chained(c, "amg_coarse_cvt", k_amg_copy<double, float>, eb, 256, 0, n, l.u.get(), l.uf.get(), active);
       return;
     }
     AmgLevel& nx = L[k + 1];
     set_ssor_params(l.smoother.get(), 1.0, 1.85, 1);
     l.smoother->apply_f32(l.ff.get(), l.uf.get(), active);
-    RSG_LAUNCH(c, "amg_zero", k_amg_zero<float>, blocks_for(nx.A->n, 256), 256, 0, nx.A->n, nx.uf.get(), active);
-    RSG_LAUNCH(c, "amg_resid", k_amg_resid<float>, eb, 256, 0, n, l.A->rowptr.get(), l.A->col.get(), l.valf.get(),
+    launch_chained(c, "amg_zero", k_amg_zero<float>, blocks_for(nx.A->n, 256), 256, 0, nx.A->n, nx.uf.get(), active);
+    launch_chained(c, "amg_resid", k_amg_resid<float>, eb, 256, 0, n, l.A->rowptr.get(), l.A->col.get(), l.valf.get(),
                l.uf.get(), l.ff.get(), l.rf.get(), active);
-    RSG_LAUNCH(c, "amg_restrict", k_amg_restrict<float>, blocks_for(l.c, 256), 256, 0, l.c, l.qptr.get(),
+    launch_chained(c, "amg_restrict", k_amg_restrict<float>, blocks_for(l.c, 256), 256, 0, l.c, l.qptr.get(),
                l.qrow.get(), l.qvalf.get(), l.rf.get(), nx.ff.get(), active);
     cycle_f32(k + 1, active);
-    RSG_LAUNCH(c, "amg_prolong", k_amg_prolong<float>, eb, 256, 0, n, l.prp.get(), l.pcol.get(), l.pvalf.get(),
+    launch_chained(c, "amg_prolong", k_amg_prolong<float>, eb, 256, 0, n, l.prp.get(), l.pcol.get(), l.pvalf.get(),
                nx.uf.get(), l.uf.get(), active);
     set_ssor_params(l.smoother.get(), 1.85, 1.0, 1);
     l.smoother->apply_f32(l.ff.get(), l.uf.get(), active);
@@ -959,10 +965,10 @@ struct AMGPrecond : Precond {
     if (!f32_ready) build_f32();
     const int n = L[0].A->n;
     const int eb = blocks_for(n, 256);
-    RSG_LAUNCH(c, "amg_zero", k_amg_zero<float>, eb, 256, 0, n, L[0].uf.get(), active);
-    RSG_LAUNCH(c, "amg_copy", (k_amg_copy<float, float>), eb, 256, 0, n, b, L[0].ff.get(), active);
+    launch_chained(c, "amg_zero", k_amg_zero<float>, eb, 256, 0, n, L[0].uf.get(), active);
+    launch_chained(c, "amg_copy", k_amg_copy<float, float>, eb, 256, 0, n, b, L[0].ff.get(), active);
     cycle_f32(0, active);
-    RSG_LAUNCH(c, "amg_copy", (k_amg_copy<float, float>), eb, 256, 0, n, L[0].uf.get(), x, active);
+    launch_chained(c, "amg_copy", k_amg_copy<float, float>, eb, 256, 0, n, L[0].uf.get(), x, active);
   }
 
   void apply(const double* b, double* x, const int* active) override { run(b, x, active, false); }

@@ -22,7 +22,8 @@
 // rows (slices) and 20 us on average on the three coarse levels (a warp per
 // row; 34 us with the ordered sum), against 245 us on average on one 8-CTA
 // cluster with a barrier per level.  That solve with its setup: 58 ms (72 with
-// the ordered sums) against 285.
+// the ordered sums) against 285; 49 with the V-cycle's 34 kernels launched as a
+// chain, a sweep readying its shared memory beside the end of the kernel before.
 #include <mutex>
 
 #include "dataflow.cuh"
@@ -120,11 +121,12 @@ __device__ __forceinline__ void await(typename Sentinel<T>::Bits (&u)[N], const 
 
 template <typename T, bool BWD>
 __global__ void __launch_bounds__(FLOW_THREADS<T>, 1) k_ssor_slices(SsorArgs<T> a) {
-  if (a.active && *a.active != 0) return;
   using S = Sentinel<T>;
   extern __shared__ __align__(16) unsigned char smem[];
   T* fresh = reinterpret_cast<T*>(smem);
   for (int i = threadIdx.x; i < a.n; i += blockDim.x) fresh[i] = S::value(S::bits);
+  chain_begin();
+  if (a.active && *a.active != 0) return;
   __syncthreads();
   const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   // Slices in order, every nwarps-th a warp's: the first one not finished
@@ -196,16 +198,16 @@ __global__ void __launch_bounds__(FLOW_THREADS<T>, 1) k_ssor_slices(SsorArgs<T> 
 
 template <typename T, bool BWD, bool SMEM>
 __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a) {
-  if (a.active && *a.active != 0) return;
   using S = Sentinel<T>;
   constexpr unsigned ALL = 0xffffffffu;
   constexpr bool TREE = sizeof(T) == 4;
   extern __shared__ __align__(16) unsigned char smem[];
   T* fresh = SMEM ? reinterpret_cast<T*>(smem) : a.out;
-  if (SMEM) {
+  if (SMEM)
     for (int i = threadIdx.x; i < a.n; i += blockDim.x) fresh[i] = S::value(S::bits);
-    __syncthreads();
-  }
+  chain_begin();
+  if (a.active && *a.active != 0) return;
+  if (SMEM) __syncthreads();
   const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   // Rows in order: in one CTA every nwarps-th is a warp's, else from a
   // counter.  Either way the first row not finished reads finished rows only,
@@ -312,6 +314,7 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
 
 template <typename T>
 __global__ void k_flow_reset(int n, T* out, unsigned* ticket, const int* active) {
+  chain_begin();
   if (active && *active != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = Sentinel<T>::value(Sentinel<T>::bits);
@@ -339,18 +342,18 @@ template <typename T, bool BWD>
 void launch_slices(Context& ctx, const char* name, const SsorArgs<T>& a) {
   static std::once_flag once;
   flow_smem(once, k_ssor_slices<T, BWD>);
-  RSG_LAUNCH(ctx, name, (k_ssor_slices<T, BWD>), 1, FLOW_THREADS<T>, sizeof(T) * a.n, a);
+  launch_chained(ctx, name, k_ssor_slices<T, BWD>, 1, FLOW_THREADS<T>, sizeof(T) * a.n, a);
 }
 
 template <typename T, bool BWD>
 void launch_rows(Context& ctx, const char* name, const SsorArgs<T>& a) {
   if (a.n <= FLOW_ROWS_MAX) {
-    RSG_LAUNCH(ctx, name, (k_ssor_rows<T, BWD, true>), 1, FLOW_ROW_THREADS, sizeof(T) * a.n, a);
+    launch_chained(ctx, name, k_ssor_rows<T, BWD, true>, 1, FLOW_ROW_THREADS, sizeof(T) * a.n, a);
     return;
   }
-  RSG_LAUNCH(ctx, name, k_flow_reset<T>, blocks_for(a.n, 256), 256, 0, a.n, a.out, a.ticket, a.active);
+  launch_chained(ctx, name, k_flow_reset<T>, blocks_for(a.n, 256), 256, 0, a.n, a.out, a.ticket, a.active);
   const int grid = std::min(ctx.num_sms, blocks_for((int64_t)a.n * 32, FLOW_ROW_THREADS));
-  RSG_LAUNCH(ctx, name, (k_ssor_rows<T, BWD, false>), grid, FLOW_ROW_THREADS, 0, a);
+  launch_chained(ctx, name, k_ssor_rows<T, BWD, false>, grid, FLOW_ROW_THREADS, 0, a);
 }
 
 }  // namespace
