@@ -202,45 +202,31 @@ __device__ void run_epilogue(int epi, KState* s, const double* t, double* hist, 
   }
 }
 
-// Block-wide deterministic sum of K values (one or two), then last-block finish.
-//
-// A double-precision warp instruction holds its sub-partition for 64 cycles
-// whatever its active lanes, so the sums are laid out for few of them in a
-// row: the block's values go through shared memory to four warps, one per
-// sub-partition, which share the quantities, add 2 K values per lane and then
-// reduce by shuffles (700 cycles for K = 2; eight warps that shuffle both
-// quantities and a thread that adds their sums took 2300, and a block of 256
-// rows pays it for each of them; see Solver::vblk).  The state that the
+// Block-wide deterministic sum of K values, then last-block finish.  A
+// double-precision warp instruction holds its sub-partition for 64 to 100
+// cycles whatever its active lanes, so the sums over the warps' values are
+// done for all quantities at once, a lane each, instead of one after the other
+// by a thread (and in the last block by every warp).  The state that the
 // epilogue reads is loaded before the last sums.
 template <int K>
 __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, int epi, KState* s, double* hist,
                               GmresDev g, int k) {
-  static_assert(K == 1 || K == 2, "four warps share the quantities");
-  constexpr int W = 4 / K;  // warps per quantity
-  __shared__ double sh[K][RT], sums[K][W];
+  __shared__ double sh[K][RT / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int mine = w / W, at = (w % W) * 32 + lane;  // of the first four warps
-#pragma unroll
-  for (int q = 0; q < K; ++q) sh[q][threadIdx.x] = v[q];
-  __syncthreads();
-  auto warp_sum = [&](double x) {
+  auto warp_sum = [&](int q, double x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sums[mine][w % W] = x;
+    if (lane == 0) sh[q][w] = x;
   };
   auto total = [&](int q) {
-    double x = sums[q][0];
+    double x = 0;
 #pragma unroll
-    for (int i = 1; i < W; ++i) x += sums[q][i];
+    for (int i = 0; i < RT / 32; ++i) x += sh[q][i];
     return x;
   };
-  if (w < 4) {
-    double x = sh[mine][at];
 #pragma unroll
-    for (int i = 32 * W; i < RT; i += 32 * W) x += sh[mine][at + i];
-    warp_sum(x);
-  }
+  for (int q = 0; q < K; ++q) warp_sum(q, v[q]);
   __syncthreads();
   if (w == 0) {
     if (lane < K) {
@@ -255,17 +241,19 @@ __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, in
   __threadfence();
   KState c;
   if (threadIdx.x == 0) c = *s;
-  if (w < 4) {
+#pragma unroll
+  for (int q = 0; q < K; ++q) {
     double x = 0;
-#pragma unroll 4
-    for (int b = at; b < (int)gridDim.x; b += 32 * W) x += __ldcg(part + mine * gridDim.x + b);
-    warp_sum(x);
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += RT) x += __ldcg(part + q * gridDim.x + b);
+    warp_sum(q, x);
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t[K];
+  if (w != 0) return;
+  const double mine = total(min(lane, K - 1));
+  double t[K];
 #pragma unroll
-    for (int q = 0; q < K; ++q) t[q] = total(q);
+  for (int q = 0; q < K; ++q) t[q] = __shfl_sync(0xffffffffu, mine, q);
+  if (lane == 0) {
     *ticket = 0;
     run_epilogue(epi, &c, t, hist, g, k);
     *s = c;
@@ -661,10 +649,7 @@ struct Solver {
   DeviceBuffer<unsigned> ticket_in;
   DeviceBuffer<KState> state_in;
   KState* hstate = nullptr;  // pinned mirror
-  // Blocks of the kernels with reductions: SpMV (eight resident per SM) and
-  // vectors.  More would be further rounds of the block's sums: 16 of the 30 us
-  // of an update of 524,288 rows went there with a block per 256 rows.
-  int nblk = 0, vblk = 0;
+  int nblk = 0;
   Csr* setup_for = nullptr;
 
   Solver(Context* c, int m, int p) : ctx(c), method(m), pc_kind(p) {
@@ -688,8 +673,7 @@ struct Solver {
       b->resize(n);
       RSG_CUDA(cudaMemsetAsync(b->get(), 0, sizeof(double) * n, ctx->stream));
     }
-    nblk = std::max(1, std::min(blocks_for(n, RT), 8 * ctx->num_sms));
-    vblk = std::max(1, std::min(blocks_for(n, RT), 4 * ctx->num_sms));
+    nblk = std::max(1, std::min(blocks_for(n, RT), 16384));
     part.resize((size_t)4 * nblk);
   }
 
@@ -771,11 +755,11 @@ struct Solver {
         pc->apply(p, ph, act);
         launch_chained(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), ph, v, rt, red(), (int)EPI_BICG_ALPHA);
-        launch_chained(*ctx, "bicg_s", k_bicg_s, vblk, RT, 0, n, r, v, s, red());
+        launch_chained(*ctx, "bicg_s", k_bicg_s, nblk, RT, 0, n, r, v, s, red());
         pc->apply(s, sh, act);
         launch_chained(*ctx, "spmv_dot", k_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), sh, t, s, red(), (int)EPI_BICG_OMEGA);
-        launch_chained(*ctx, "bicg_update", k_bicg_update, vblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
+        launch_chained(*ctx, "bicg_update", k_bicg_update, nblk, RT, 0, n, ph, sh, s, t, rt, x, r, red());
       }
     }
   }
@@ -791,11 +775,11 @@ struct Solver {
       if (hstate->status != 0) break;
       for (int it = 0; it < batch(); ++it) {
         pc->apply(r, z, act);
-        launch_chained(*ctx, "dot", k_dot, vblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
+        launch_chained(*ctx, "dot", k_dot, nblk, RT, 0, n, r, z, red(), (int)EPI_CG_RHO, 0);
         launch_chained(*ctx, "cg_p", k_cg_p, eb, 256, 0, n, z, p, state.get());
         launch_chained(*ctx, "spmv_dot", k_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                    A.sell_col.get(), A.sell_val.get(), p, q, p, red(), (int)EPI_CG_ALPHA);
-        launch_chained(*ctx, "cg_update", k_cg_update, vblk, RT, 0, n, p, q, x, r, red());
+        launch_chained(*ctx, "cg_update", k_cg_update, nblk, RT, 0, n, p, q, x, r, red());
       }
     }
   }
@@ -837,7 +821,7 @@ struct Solver {
     // r = b - A x; monitor(|r|)
     RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
-    launch_chained(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    launch_chained(*ctx, "fgm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     for (;;) {
       read_state();
       if (hstate->status != 0) break;
@@ -846,25 +830,25 @@ struct Solver {
         const int i = hstate->gm_i;
         // z_i = M(v_i): FP32 BiCGstab + ILU(0) from zero
         launch_chained(*ctx, "inner_reset", k_inner_reset, 1, 1, 0, sin, inner_rtol, 0.0, inner_iters);
-        launch_chained(*ctx, "inner_init", k_f32_init, vblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
+        launch_chained(*ctx, "inner_init", k_f32_init, nblk, RT, 0, n, vcol(i), ir, irt, ix, ri);
         for (int q = 0; q < inner_iters; ++q) {
           launch_chained(*ctx, "inner_p", k_f32_bicg_p, eb, 256, 0, n, ir, iv, ip, sin);
           pc->apply_f32(ip, iph, act_in);
           launch_chained(*ctx, "inner_spmv_dot", k_f32_spmv_dot<1>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), iph, iv, irt, ri, (int)EPI_BICG_ALPHA);
-          launch_chained(*ctx, "inner_s", k_f32_bicg_s, vblk, RT, 0, n, ir, iv, is, ri);
+          launch_chained(*ctx, "inner_s", k_f32_bicg_s, nblk, RT, 0, n, ir, iv, is, ri);
           pc->apply_f32(is, ish, act_in);
           launch_chained(*ctx, "inner_spmv_dot", k_f32_spmv_dot<2>, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(),
                      A.sell_col.get(), A.sell_valf.get(), ish, it, is, ri, (int)EPI_BICG_OMEGA);
-          launch_chained(*ctx, "inner_update", k_f32_bicg_update, vblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
+          launch_chained(*ctx, "inner_update", k_f32_bicg_update, nblk, RT, 0, n, iph, ish, is, it, irt, ix, ir, ri);
         }
         launch_chained(*ctx, "to_f64", k_f32_to_f64, eb, 256, 0, n, ix, zcol(i), (const KState*)sin, state.get());
         // w = A z_i, then the Arnoldi step of GMRES.java:146-162 on w
         launch_spmv(*ctx, A, zcol(i), w, nullptr);
         for (int k2 = 0; k2 <= i; ++k2)
-          launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
+          launch_chained(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, k2 > 0 ? vcol(k2 - 1) : (const double*)nullptr,
                      vcol(k2), red(), k2, (int)EPI_GM_H);
-        launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        launch_chained(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
         launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
@@ -875,7 +859,7 @@ struct Solver {
       RSG_LAUNCH(*ctx, "fgm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                  A.sell_val.get(), x, b, r, (double*)nullptr, red(), (int)EPI_NONE);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      launch_chained(*ctx, "fgm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      launch_chained(*ctx, "fgm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 
@@ -895,7 +879,7 @@ struct Solver {
     RSG_LAUNCH(*ctx, "gm_resid", k_resid, nblk, RT, 0, n, A.slice_base.get(), A.row_len.get(), A.sell_col.get(),
                A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
     pc->apply(u, r, nullptr);
-    launch_chained(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+    launch_chained(*ctx, "gm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     pc->apply(b, u, nullptr);
     for (;;) {
       read_state();
@@ -907,9 +891,9 @@ struct Solver {
         launch_spmv(*ctx, A, vcol(i), u, nullptr);
         pc->apply(u, w, nullptr);
         for (int k = 0; k <= i; ++k)
-          launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
+          launch_chained(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, k > 0 ? vcol(k - 1) : (const double*)nullptr,
                      vcol(k), red(), k, (int)EPI_GM_H);
-        launch_chained(*ctx, "gm_mgs", k_gm_mgs, vblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
+        launch_chained(*ctx, "gm_mgs", k_gm_mgs, nblk, RT, 0, n, w, vcol(i), (const double*)nullptr, red(), i + 1,
                    (int)EPI_GM_NORMW);
         launch_chained(*ctx, "gm_vset", k_gm_vset, eb, 256, 0, n, w, vcol(i + 1), state.get());
         read_state();
@@ -922,7 +906,7 @@ struct Solver {
                  A.sell_val.get(), x, b, u, (double*)nullptr, red(), (int)EPI_NONE);
       pc->apply(u, r, nullptr);
       RSG_LAUNCH(*ctx, "iter_inc", k_iter_inc, 1, 1, 0, state.get());
-      launch_chained(*ctx, "gm_norm", k_dot, vblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
+      launch_chained(*ctx, "gm_norm", k_dot, nblk, RT, 0, n, r, r, red(), (int)EPI_GM_OUTER, 0);
     }
   }
 };
