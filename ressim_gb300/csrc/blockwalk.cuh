@@ -26,14 +26,19 @@
 // a running CTA never waits for one that has not started, whatever else
 // occupies the GPU.
 //
-// What bounds it: the chain of steps and the hops between blocks.  A step of
-// the chain takes 125 ns in double precision (four terms, 64 cycles each) and
-// about 65 in single; a value reaches the next block's chain in about 1.4 us,
-// 31 + 5 times in a row on a 128 x 128 x 32 grid.  There a walk takes 190 us
-// (double) and 128 us (single), against 700 to 780 and 480 for the level walk
-// on one 16-CTA cluster (ring.cuh), whose 506 levels each wait for a CTA
-// barrier and a load from memory; on 64 x 64 x 16, 83 and 47 us against about
-// 300 and 190.
+// What bounds it: the chain of steps and the hops between blocks, ni + 2 nj
+// steps and nk hops on a grid.  A step takes 208 ns in double precision (four
+// terms of about 100 cycles each, one after the other on the sub-partition; a
+// single block of 2048 x 32 rows never waits for anything else) and 110 in
+// single, a hop 2.2 and 1.5 us.  A walk, chained to the kernels around it,
+// double and single: 2048 x 32 x 1 445 and 239 us, 32 x 32 x 8 40 and 25, 64 x
+// 64 x 16 87 and 54, 128 x 128 x 32 190 and 128.  The level walk on one 16-CTA
+// cluster (ring.cuh), whose levels each wait for a CTA barrier and a load from
+// memory, took 700 to 780 and 480 us on the last, about 300 and 190 on the one
+// before.  Measured and not kept: handing the chain's newest operands on by
+// shuffles (204 ns a step: the terms bound it, not their exchange), staging
+// further ahead, more or fewer warps of a kind, fetch warps that take two steps
+// in a row (a quarter slower in three dimensions) or release steps together.
 //
 // A row's sum starts from the right-hand side and subtracts fused products;
 // upper factors are stored divided by their row's diagonal (with its
