@@ -653,6 +653,9 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bw_addr(&bars) + 8 * (threadIdx.x - 32)),
                  "r"(threadIdx.x - 32 < BW_STAGES_MAX ? 33 : 1)  // coef: the bulk copies' issuer and every lane's own copy
                  : "memory");
+  // the barriers' initialisation is visible to the bulk copies
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
   const int blk = (int)(sh_ticket & 0x7fffffffu), which = (int)(sh_ticket >> 31);
   const int s0 = g.blk_step[blk], nst = g.blk_step[blk + 1] - s0;
