@@ -419,22 +419,26 @@ __device__ __forceinline__ bool bw_test(const unsigned long long* bar, unsigned 
       : "memory");
   return ok != 0;
 }
-// Waits for a phase, the whole warp together.  A wait that is given up goes
-// on with what is there, so that every warp ends; the walk is then reported
-// as failed.
-__device__ __forceinline__ void bw_wait(const unsigned long long* bar, unsigned parity, int* err) {
+__device__ __forceinline__ bool bw_try(const unsigned long long* bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bw_addr(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok);
+}
+// Waits for a phase, the whole warp together.  False when the wait is given
+// up: the walk has then failed, and the warp ends at once, because what it
+// waited for (staged indices among it) is not there to be used.  The warps
+// that wait for this one in turn give up by the error that is set.
+__device__ __forceinline__ bool bw_wait(const unsigned long long* bar, unsigned parity, int* err) {
   unsigned long long start = 0;
   for (int i = 1;; ++i) {
-    unsigned ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bw_addr(bar)), "r"(parity)
-        : "memory");
-    if (__all_sync(0xffffffffu, ok)) return;
+    if (bw_try(bar, parity)) return true;
     if ((i & 255) == 0 && __any_sync(0xffffffffu, wait_over(start, err))) {
       atomicCAS(err, 0, 1);
-      return;
+      return false;
     }
   }
 }
@@ -569,7 +573,7 @@ __device__ __forceinline__ void bw_chain(const BlockWalkArgs& g, const BwStage<T
   Terms a, b, c;
 #pragma unroll 1
   for (int s = 0; s < nst;) {
-    bw_wait(&bars.part[s & (D - 1)], s / D & 1, g.err);
+    if (!bw_wait(&bars.part[s & (D - 1)], s / D & 1, g.err)) return;
     load(a, s);
 #pragma unroll
     for (int q = 0; q < NP; ++q) a.v = fma(-a.ap[q], xs[a.ix.i[q]], a.v);
@@ -604,7 +608,7 @@ __device__ __forceinline__ void bw_chain_wide(const BlockWalkArgs& g, const BwSt
 #pragma unroll 1
   for (int s = 0; s < nst; ++s) {
     unsigned char* sp = smem + (s & (D - 1)) * z.SS;
-    bw_wait(&bars.part[s & (D - 1)], s / D & 1, g.err);
+    if (!bw_wait(&bars.part[s & (D - 1)], s / D & 1, g.err)) return;
     const T v = bw_terms(reinterpret_cast<const T*>(sp + z.IS + z.VS)[32 + lane],
                          reinterpret_cast<const T*>(sp + z.IS) + (g.w.old + g.w.fresh) * 32 + lane,
                          reinterpret_cast<const BwIdx*>(sp) + g.w.early_groups() * 32 + lane, xs, g.w.pre + g.w.last);
@@ -671,20 +675,22 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
   }
   if ((warp & 3) == 0) return;
   const int role = warp - 1 - (warp >> 2);
-  auto wait_done = [&](int s) { bw_wait(&bars.done[s & (D - 1)], s / D & 1, g.err); };
+  auto wait_done = [&](int s) { return bw_wait(&bars.done[s & (D - 1)], s / D & 1, g.err); };
+  auto wait_coef = [&](int s) { return bw_wait(&bars.coef[s & (D - 1)], s / D & 1, g.err); };
+  auto wait_full = [&](int s) { return bw_wait(&bars.full[s & (D - 1)], s / D & 1, g.err); };
   if (role < BW_EARLY) {
     for (int s = role; s < nst; s += BW_EARLY) {
       unsigned char* sp = smem + (s & (D - 1)) * z.SS;
-      bw_wait(&bars.coef[s & (D - 1)], s / D & 1, g.err);
+      if (!wait_coef(s)) return;
       const T* val = reinterpret_cast<const T*>(sp + z.IS) + lane;
       const BwIdx* idx = reinterpret_cast<const BwIdx*>(sp) + lane;
       T* bp = reinterpret_cast<T*>(sp + z.IS + z.VS) + lane;
       T v = bp[0];
       if (UPPER) v *= val[g.w.total() * 32];
-      if (s >= BW_NEW) bw_wait(&bars.full[(s - BW_NEW) & (D - 1)], (s - BW_NEW) / D & 1, g.err);
-      if (g.own_old && s >= BW_OLD) wait_done(s - BW_OLD);
+      if (s >= BW_NEW && !wait_full(s - BW_NEW)) return;
+      if (g.own_old && s >= BW_OLD && !wait_done(s - BW_OLD)) return;
       v = bw_terms(v, val, idx, xs, g.w.old);
-      bw_wait(&bars.full[s & (D - 1)], s / D & 1, g.err);
+      if (!wait_full(s)) return;
       v = bw_terms(v, val + g.w.old * 32, idx + g.w.old_groups() * 32, xs, g.w.fresh);
       bp[32] = v;
       bw_arrive(&bars.part[s & (D - 1)], lane);
@@ -704,9 +710,10 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
       if (row >= 0) io.x[row] = v;
       __syncwarp();
     };
-    int s = f;
+    bool ok = true;
+    int s = f, issued = -1;
     for (; s < nst; s += BW_STREAM) {
-      if (s >= D - BW_NEW) wait_done(s - D + BW_NEW);
+      if (s >= D - BW_NEW && !(ok = wait_done(s - D + BW_NEW))) break;
       if (s >= D) retire(s - D);
       // Indices of the right-hand side: a load from global memory here, even
       // of several steps ahead, would have each step wait for it (loads of
@@ -714,7 +721,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
       int bi;
       if (s < BW_BACK) bi = g.bsrc[(size_t)(s0 + s) * BW_LANES + lane];
       else {
-        bw_wait(&bars.coef[(s - BW_BACK) & (D - 1)], (s - BW_BACK) / D & 1, g.err);
+        if (!(ok = wait_coef(s - BW_BACK))) break;
         bi = reinterpret_cast<const int*>(smem + ((s - BW_BACK) & (D - 1)) * z.SS + g.w.index_bytes())[lane];
       }
       unsigned char* sp = smem + (s & (D - 1)) * z.SS;
@@ -728,13 +735,20 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
         cp_bulk(sp, g.ints + (size_t)(s0 + s) * z.IS, z.IS, bar);
         cp_bulk(sp + z.IS, reinterpret_cast<const unsigned char*>(io.vals) + (size_t)(s0 + s) * z.VS, z.VS, bar);
       }
+      issued = s;
       for (int r = r0 + s * rs + lane; r < min(r1, r0 + (s + 1) * rs); r += 32) S::store(reset + r, S::bits);
     }
     if (UPPER)
-      for (; s - D < nst; s += BW_STREAM)
-        if (s >= D) {
-          wait_done(s - D);
-          retire(s - D);
+      for (; ok && s - D < nst; s += BW_STREAM)
+        if (s >= D && (ok = wait_done(s - D))) retire(s - D);
+    // A walk given up: the copies in flight land before the CTA may end.
+    // Their barriers take this warp's arrivals alone, so the wait has an end;
+    // otherwise the early warps have waited for every step's.
+    if (!ok)
+      for (int q = issued; q >= 0 && q > issued - D; q -= BW_STREAM)
+        for (unsigned long long start = 0;;) {
+          if (bw_try(&bars.coef[q & (D - 1)], q / D & 1)) break;
+          if (__any_sync(0xffffffffu, time_over(start))) break;
         }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
@@ -755,7 +769,7 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
       const int h0 = h0_n, h1 = h1_n;
       const int hr[2] = {hr_n[0], hr_n[1]};
       ahead(s + BW_FETCH);
-      bw_wait(&bars.coef[s & (D - 1)], s / D & 1, g.err);  // not ahead of the coefficients: the window is bounded
+      if (!wait_coef(s)) return;  // not ahead of the coefficients: the window is bounded
       for (int q = 0; h0 + 32 * q < h1; ++q) {
         const int h = h0 + lane + 32 * q;
         const bool mine = h < h1;
@@ -769,13 +783,13 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
           if (mine && v == S::bits) v = S::load(p);
           if ((i & 255) == 0 && __any_sync(0xffffffffu, wait_over(start, g.err))) {
             atomicCAS(g.err, 0, 1 + s);
-            break;
+            return;
           }
         }
         if (mine) hs[(h - hbase) & (g.halo - 1)] = S::value(v);
       }
       // released in order: a step's operands may have been staged with an earlier step
-      if (s > 0) bw_wait(&bars.full[(s - 1) & (D - 1)], (s - 1) / D & 1, g.err);
+      if (s > 0 && !wait_full(s - 1)) return;
       bw_arrive(&bars.full[s & (D - 1)], lane);
     }
   }

@@ -55,13 +55,18 @@ __global__ void k_sentinel(int64_t n, T* x) {
 // Nanoseconds a wait may take: far more than a kernel, also among others.
 constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;
 
-// Whether a wait is to be given up, asked now and then (start: 0 at first):
-// it has taken too long, or some other wait has.
-__device__ __forceinline__ bool wait_over(unsigned long long& start, const int* err) {
+// Whether a wait that began at `start` (0 at first) has taken too long.
+__device__ __forceinline__ bool time_over(unsigned long long& start) {
   unsigned long long t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   if (!start) start = t;
-  return t - start > WAIT_LIMIT_NS || *(const volatile int*)err;
+  return t - start > WAIT_LIMIT_NS;
+}
+
+// Whether a wait is to be given up, asked now and then: it has taken too
+// long, or some other wait has.
+__device__ __forceinline__ bool wait_over(unsigned long long& start, const int* err) {
+  return time_over(start) || *(const volatile int*)err;
 }
 
 }  // namespace rsg
