@@ -741,15 +741,14 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
     if (UPPER)
       for (; ok && s - D < nst; s += BW_STREAM)
         if (s >= D && (ok = wait_done(s - D))) retire(s - D);
-    // A walk given up: the copies in flight land before the CTA may end.
-    // Their barriers take this warp's arrivals alone, so the wait has an end;
-    // otherwise the early warps have waited for every step's.
-    if (!ok)
-      for (int q = issued; q >= 0 && q > issued - D; q -= BW_STREAM)
-        for (unsigned long long start = 0;;) {
-          if (bw_try(&bars.coef[q & (D - 1)], q / D & 1)) break;
-          if (__any_sync(0xffffffffu, time_over(start))) break;
-        }
+    // The copies land before the CTA may end, also when the warps that use
+    // them have given up.  Their barriers take this warp's arrivals alone, so
+    // the wait has an end.
+    for (int q = issued; q >= 0 && q > issued - D; q -= BW_STREAM)
+      for (unsigned long long start = 0;;) {
+        if (bw_try(&bars.coef[q & (D - 1)], q / D & 1)) break;
+        if (__any_sync(0xffffffffu, time_over(start))) break;
+      }
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
     const int f = role - BW_EARLY - BW_STREAM;
