@@ -334,6 +334,7 @@ __global__ void __launch_bounds__(128) k_seg_sort(int n, const int* __restrict__
       for (int c = 0; c < SORT_CHUNKS; ++c) place[c] += other < k[c];
     }
   }
+  __syncwarp();  // every lane has read its entries before any place is written (shuffles order no memory)
 #pragma unroll
   for (int c = 0; c < SORT_CHUNKS; ++c)
     if (32 * c + lane < len) {

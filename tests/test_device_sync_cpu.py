@@ -32,3 +32,13 @@ def test_mbarriers_are_fenced_before_use(path):
         assert "fence.mbarrier_init" in between
         if "cp.async.bulk" in src:
             assert "fence.proxy.async" in between
+
+
+def test_segment_sort_reads_before_it_writes():
+    """k_seg_sort (amg.cu) puts a segment back in place, a lane's entries where
+    other lanes read theirs: a warp barrier stands between."""
+    src = code(os.path.join(CSRC, "amg.cu"))
+    body = src[src.index("k_seg_sort(int n"):]
+    body = body[:body.index("\n}")]
+    read, write = body.rindex("val[p0 + e]"), body.rindex("key[p0 + place[c]] =")
+    assert read < body.index("__syncwarp()", read) < write
