@@ -1268,6 +1268,13 @@ void ILUPrecond::trans_apply(const double* b, double* x, const int* active) {
     // part, transposed); L^T is upper triangular.
     build_plan(T.At, T.Ut, false, 0, true);
     build_plan(T.At, T.Lt, true, 1, false);
+    // ring schedules, for 16 CTAs where there is one: 64x64x16 397 and 477 us a
+    // sweep, 990 and 1,180 on the cluster that meets at a barrier per level
+    for (int u = 0; u < 2; ++u) {
+      HostRing H[2] = {host_ring(T.At, u == 1, 0), HostRing()};
+      if (!H[0].C) H[1] = host_ring(T.At, u == 1, 1);
+      upload_rings(T.At, u == 0 ? T.Ut : T.Lt, H, u == 0);
+    }
     T.built = true;
   }
   RSG_LAUNCH(*ctx, "ilu_trans_gather", k_gather_vals, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, T.tsrc.get(),
