@@ -591,9 +591,9 @@ rsg_status rsg_ensemble_step(int32_t count, rsg_sim* const* sims, const double* 
 /* Ensembles: one time step of dt[i] on every member, with the pressure solver
  * that `precision` names.  Each member's Discretisation.solve(dt)
  * (numerics/Discretisation.java:208-225) runs as in rsg_sim_step.  A member
- * with a context of its own whose ILU(0) factors have block walks is stepped
- * on its own stream, from one of up to as many host threads as the machine
- * has.  The others go in lockstep: they assemble their Jacobians and factor
+ * whose ILU(0) factors have block walks is stepped on a stream of its own, from
+ * one of up to as many host threads as the machine has.  The others go in
+ * lockstep: they assemble their Jacobians and factor
  * their ILU(0) preconditioners, then ONE persistent kernel of thread-block
  * clusters takes them from a work queue and solves each pressure system
  * completely (BiCGstab, mtj/.../sparse/BiCGstab.java:65-116, with ILU(0))
@@ -607,8 +607,9 @@ rsg_status rsg_ensemble_step(int32_t count, rsg_sim* const* sims, const double* 
  * step fails stops there (statuses[i], infos[i]); the others go on.  Returns
  * the first failing member's status.  Results agree with rsg_sim_step per
  * member to the Krylov solver's rounding (the dot products are summed in a
- * different order) and do not depend on the number of members or on their
- * order.  No counterpart in the reference (RS runs one field per process). */
+ * different order) and do not depend on the number of members, on their order
+ * or on whether they share a context.  No counterpart in the reference (RS
+ * runs one field per process). */
 rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const double* dt, int32_t precision,
                                      rsg_step_info* infos, int32_t* statuses);
 /* IterativeSolver.solve (mtj/.../sparse/IterativeSolver.java:43-74) on many

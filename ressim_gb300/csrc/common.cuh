@@ -89,6 +89,11 @@ struct Context {
   // set by kernels whose bounded waits ran out (1 + site); read after solves
   DeviceBuffer<int> dev_err;
 
+  void open();   // stream, staging page, error flag; device and num_sms are set
+  void close();  // gives them back
+  // Takes over what another context, standing in for this one, has counted.
+  void take_counts(Context& other);
+
   cudaEvent_t get_event();
   void flush_profile();  // requires a synchronized stream
   void sync();

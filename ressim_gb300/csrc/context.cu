@@ -5,6 +5,39 @@
 
 namespace rsg {
 
+void Context::open() {
+  RSG_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+  RSG_CUDA(cudaMallocHost(&pinned, 4096));
+  dev_err.resize(1);
+  RSG_CUDA(cudaMemsetAsync(dev_err.get(), 0, sizeof(int), stream));
+}
+
+void Context::close() {
+  cudaSetDevice(device);
+  if (stream) cudaStreamSynchronize(stream);
+  for (auto& p : pending) {
+    cudaEventDestroy(p.a);
+    cudaEventDestroy(p.b);
+  }
+  for (auto e : event_pool) cudaEventDestroy(e);
+  for (auto e : timers)
+    if (e) cudaEventDestroy(e);
+  if (pinned) cudaFreeHost(pinned);
+  if (stream) cudaStreamDestroy(stream);
+  stream = nullptr;
+}
+
+void Context::take_counts(Context& other) {
+  launches += other.launches;
+  other.launches = 0;
+  for (auto& kv : other.profile) {
+    auto& e = profile[kv.first];
+    e.ms += kv.second.ms;
+    e.launches += kv.second.launches;
+  }
+  other.profile.clear();
+}
+
 cudaEvent_t Context::get_event() {
   if (!event_pool.empty()) {
     cudaEvent_t e = event_pool.back();
@@ -91,10 +124,7 @@ rsg_status rsg_context_create(int32_t device, rsg_ctx** out) {
     RSG_CUDA(cudaSetDevice(device));
     h->c.device = device;
     h->c.num_sms = prop.multiProcessorCount;
-    RSG_CUDA(cudaStreamCreateWithFlags(&h->c.stream, cudaStreamNonBlocking));
-    RSG_CUDA(cudaMallocHost(&h->c.pinned, 4096));
-    h->c.dev_err.resize(1);
-    RSG_CUDA(cudaMemsetAsync(h->c.dev_err.get(), 0, sizeof(int), h->c.stream));
+    h->c.open();
   });
   if (st != RSG_OK) {
     delete h;
@@ -106,17 +136,7 @@ rsg_status rsg_context_create(int32_t device, rsg_ctx** out) {
 
 rsg_status rsg_context_destroy(rsg_ctx* ctx) {
   if (!ctx) return RSG_BAD_ARG;
-  cudaSetDevice(ctx->c.device);
-  cudaStreamSynchronize(ctx->c.stream);
-  for (auto& p : ctx->c.pending) {
-    cudaEventDestroy(p.a);
-    cudaEventDestroy(p.b);
-  }
-  for (auto e : ctx->c.event_pool) cudaEventDestroy(e);
-  for (auto e : ctx->c.timers)
-    if (e) cudaEventDestroy(e);
-  if (ctx->c.pinned) cudaFreeHost(ctx->c.pinned);
-  if (ctx->c.stream) cudaStreamDestroy(ctx->c.stream);
+  ctx->c.close();
   delete ctx;
   return RSG_OK;
 }

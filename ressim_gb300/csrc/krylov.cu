@@ -939,8 +939,13 @@ void solver_solve(Solver& s, Csr& A, const double* b, double* x, rsg_solve_info*
 void solver_solve_member(Solver& s, Csr& A, const double* b, double* x, int precision, rsg_solve_info* info) {
   s.solve(A, b, x, info, precision ? RSG_FGMRES_MIXED : RSG_BICGSTAB);
 }
+bool solver_suits_ensembles(Solver& s) { return s.method == RSG_BICGSTAB && s.pc_kind == RSG_PC_ILU; }
 bool solver_runs_alone(Solver& s, int precision) {
-  return s.method == RSG_BICGSTAB && s.pc_kind == RSG_PC_ILU && ilu_has_block_walks(s.pc.get(), precision != 0);
+  return solver_suits_ensembles(s) && ilu_has_block_walks(s.pc.get(), precision != 0);
+}
+void solver_use(Solver& s, Context* c) {
+  s.ctx = c;
+  s.pc->use(c);
 }
 
 SolverView solver_view(Solver& s) {

@@ -110,6 +110,9 @@ struct Precond {
   // x := M^{-1} b (x may be read as the starting iterate, as SSOR does)
   virtual void apply(const double* b, double* x, const int* active) = 0;
   virtual void trans_apply(const double* b, double* x, const int* active) = 0;
+  // From now on its work goes to this context's stream (ILU(0) only; what was
+  // queued on the other has ended).
+  virtual void use(Context* c) {}
   // called once before a solve's applies (f32: before its apply_f32 calls)
   virtual void begin_solve(bool f32) {}
   // Preconditioner.apply with MTJ's rounding (the solvers' applies may fuse
@@ -139,10 +142,13 @@ SolverPtr make_solver(Context* ctx, int method, int precond, double rtol, double
 void solver_setup(Solver& s, Csr& A);
 void solver_solve(Solver& s, Csr& A, const double* b, double* x, rsg_solve_info* info);
 void solver_set_inner(Solver& s, int iterations, double rtol);
-// An ensemble member's pressure solve on its own stream: whether its solver
-// (BiCGstab + ILU(0)) has block walks for the precision, and the solve
+// An ensemble member's pressure solve on its own stream: whether its solver is
+// one that ensembles take (BiCGstab + ILU(0)), whether that has block walks
+// for the precision after its setup, the stream to use, and the solve
 // (precision 0: BiCGstab, 1: the mixed-precision method) as solver_solve.
+bool solver_suits_ensembles(Solver& s);
 bool solver_runs_alone(Solver& s, int precision);
+void solver_use(Solver& s, Context* c);
 void solver_solve_member(Solver& s, Csr& A, const double* b, double* x, int precision, rsg_solve_info* info);
 // what a solver was created with, and its preconditioner
 struct SolverView {

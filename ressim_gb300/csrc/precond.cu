@@ -970,6 +970,7 @@ struct ILUPrecond : Precond {
   DeviceBuffer<int> flag, upd_ptr, upd_l, upd_j;
   const int* pattern_id = nullptr;
   explicit ILUPrecond(Context* c) : ctx(c) {}
+  void use(Context* c) override { ctx = walk.ctx = c; }
 
   // elimination program of the level-by-level factorisation (see FactorArgs)
   void elimination_program(Csr& M) {

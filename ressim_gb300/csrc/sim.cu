@@ -1424,8 +1424,19 @@ __global__ void k_dt_terms(SimDev d, const int* __restrict__ locked, const doubl
   atomicMax(out + 1, (unsigned long long)__double_as_longlong(t));
 }
 
+struct LaneDeleter {
+  void operator()(Context* c) const {
+    c->close();
+    delete c;
+  }
+};
+
 struct Sim {
   Context* ctx;
+  // Stands in for ctx, with a stream of its own, while ensemble members that
+  // share a context are stepped at the same time.
+  std::unique_ptr<Context, LaneDeleter> lane;
+  Context* home = nullptr;  // ctx, while the lane stands in for it
   Mesh* mesh;
   rsg_runspec spec;
   int n, nc, nconn;
@@ -1458,6 +1469,33 @@ struct Sim {
   DeviceBuffer<unsigned long long> dt_terms;
   std::vector<double> h_src_total;  // dt-independent sum of regular source rates per component
   bool keep_jacobian = false;
+
+  // Moves the simulator to its lane, and back (solvers that suit ensembles).
+  void use(Context* c) {
+    ctx = A.m.ctx = c;
+    solver_use(*solver, c);
+  }
+  void to_lane() {
+    ctx->sync();
+    if (!lane) {
+      std::unique_ptr<Context, LaneDeleter> l(new Context());
+      l->device = ctx->device;
+      l->num_sms = ctx->num_sms;
+      l->open();
+      lane = std::move(l);
+    }
+    lane->profiling = ctx->profiling;
+    home = ctx;
+    use(lane.get());
+  }
+  void to_home(bool failed) {
+    Context& c = *home;
+    home = nullptr;
+    use(&c);
+    if (failed) c.last_error = lane->last_error;
+    lane->sync();
+    c.take_counts(*lane);
+  }
 
   SimDev dev() {
     SimDev d;
@@ -2355,25 +2393,35 @@ rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const 
     if (!seen.insert(sims[i]->s.get()).second) return RSG_BAD_ARG;  // a member listed twice
   }
   std::vector<rsg_status> st(count, RSG_OK);
-  std::vector<char> live(count, 1), done(count, 0), ended(count, 0), assembled(count, 0);
+  std::vector<char> live(count, 1), done(count, 0), ended(count, 0), begun(count, 0), assembled(count, 0);
   std::vector<rsg_step_info> inf(count);
-  // Members with a context of their own and block walks run their whole step
-  // on their own stream: a block walk leaves most SMs to the other members
-  // (a 56x56x14 member's uses 28 of 152), and its chain of steps is shorter
-  // than the lockstep launch's levels.  Mixed precision, one time step: six
-  // members of 32x32x8 to 56x56x14 98 ms against 385, 64 members of up to
-  // 96x96x24 1.99 s against 6.97 (FP64: 2.25 s against 7.08).
-  // Whether a member does so depends on that member alone, so its results do
-  // not depend on the others.  The rest go on below in lockstep.
+  // A member whose solver has block walks runs its whole step on a stream of
+  // its own: its context's, or its lane's where members share a context.  A
+  // block walk leaves most SMs to the other members (a 56x56x14 member's has
+  // 42 blocks for 152 SMs), and its chain of steps is shorter than the lockstep
+  // launch's levels.  Mixed precision, one time step: six members of 32x32x8
+  // to 56x56x14 98 ms against 385, 64 members of up to 96x96x24 1.99 s against
+  // 6.97 (FP64: 2.25 s against 7.08); on one context, six 100 ms against 320
+  // and 40 of up to 56x56x14 419 against 939.  Whether a member does so depends
+  // on that member alone, so its results do not depend on the others or on who
+  // shares its context.  The rest go on below in lockstep.
   std::map<rsg::Context*, int> sharing;
   for (int i = 0; i < count; ++i) ++sharing[sims[i]->s->ctx];
   std::vector<int> own;
+  own.reserve(count);
   for (int i = 0; i < count; ++i) {
-    if (sims[i]->s->ctx->device != sims[0]->s->ctx->device) {  // members must share one device
+    rsg::Sim& m = *sims[i]->s;
+    if (m.ctx->device != sims[0]->s->ctx->device) {  // members must share one device
       st[i] = RSG_BAD_ARG;
       live[i] = 0;
-    } else if (sharing[sims[i]->s->ctx] == 1) {
-      own.push_back(i);
+    } else if (rsg::solver_suits_ensembles(*m.solver)) {
+      if (sharing[m.ctx] > 1)
+        st[i] = guarded(m.ctx, [&] {
+          RSG_CUDA(cudaSetDevice(m.ctx->device));
+          m.to_lane();
+        });
+      if (st[i] != RSG_OK) live[i] = 0;
+      else own.push_back(i);
     }
   }
   std::stable_sort(own.begin(), own.end(), [&](int a, int b) { return sims[a]->s->n > sims[b]->s->n; });
@@ -2381,6 +2429,7 @@ rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const 
     rsg::Sim& m = *sims[i]->s;
     st[i] = guarded(m.ctx, [&] {
       RSG_CUDA(cudaSetDevice(m.ctx->device));
+      begun[i] = 1;
       m.step_begin(dt[i]);
       for (;;) {
         m.newton_assemble(dt[i]);
@@ -2412,7 +2461,16 @@ rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const 
   }
   for (int i = 0; i < count; ++i) {
     rsg::Sim& m = *sims[i]->s;
-    if (!live[i] || sharing[m.ctx] == 1) continue;
+    if (!m.home) continue;
+    const rsg_status back = guarded(m.home, [&] { m.to_home(st[i] != RSG_OK); });
+    if (back != RSG_OK) {
+      if (st[i] == RSG_OK) st[i] = back;
+      live[i] = 0;
+    }
+  }
+  for (int i = 0; i < count; ++i) {
+    rsg::Sim& m = *sims[i]->s;
+    if (!live[i] || begun[i]) continue;
     st[i] = guarded(m.ctx, [&] {
       RSG_CUDA(cudaSetDevice(m.ctx->device));
       m.step_begin(dt[i]);
