@@ -23,7 +23,6 @@
 // overlapping aggregates in ascending node order (MTJ's order is that of a
 // java.util.HashSet).
 #include <algorithm>
-#include <mutex>
 #include <cmath>
 #include <string>
 
@@ -746,8 +745,8 @@ struct AMGPrecond : Precond {
       gbits.resize((n + 31) / 32);
       smem = stage;
     }
-    static std::once_flag attr;
-    std::call_once(attr, [] { cudaFuncSetAttribute(k_agg_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); });
+    static PerDevice allowed;
+    allow_smem(allowed, c, k_agg_greedy, 200 * 1024);
     RSG_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(int), c.stream));
     PhaseArgs p1{n, A.rowptr.get(), A.col.get(), S.get(), R0.get(), nullptr, a1.get(), counter.get(), gbits.get(),
                  flag.get(), 0};

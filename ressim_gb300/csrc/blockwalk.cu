@@ -2,7 +2,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <mutex>
 #include <unordered_map>
 
 #include "blockwalk.cuh"
@@ -871,10 +870,8 @@ void launch(Context& ctx, const char* name, const BlockWalk& P, const BlockWalkI
   const size_t stage = bw_int_bytes(P.w, UPPER) + (size_t)(P.w.total() + (UPPER ? 1 : 0)) * 32 * sizeof(T) + 64 * sizeof(T);
   const size_t smem = D * stage + (size_t)(BW_OWN * BW_LANES + P.halo + 2) * sizeof(T);
   auto kern = k_block_walk<T, UPPER, D>;
-  static std::once_flag once;
-  std::call_once(once, [&] {
-    RSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BW_SMEM_MAX));
-  });
+  static PerDevice allowed;
+  allow_smem(allowed, ctx, kern, BW_SMEM_MAX);
   const BlockWalkArgs g{P.blk_step.get(), P.hptr.get(), P.hsrc.get(), P.ints.get(), P.bsrc.get(), P.w, P.nblk, P.halo,
                         (int)P.own_old, P.ticket.get(), ctx.dev_err.get()};
   launch_chained(ctx, name, kern, P.nblk, BW_THREADS, smem, g, io);

@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/rsg.h"
+#include "perdevice.hpp"
 
 namespace rsg {
 
@@ -173,6 +174,16 @@ __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.launch_dependents;");
 }
 #endif
+
+// Lets `kernel` use `bytes` of dynamic shared memory on the context's device;
+// done: the kernel's own (static) record of where it may.
+template <typename Kernel>
+inline void allow_smem(PerDevice& done, const Context& ctx, Kernel kernel, size_t bytes) {
+  done.ask(ctx.device, [&] {
+    RSG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return true;
+  });
+}
 
 inline int blocks_for(int64_t n, int threads) { return (int)((n + threads - 1) / threads); }
 

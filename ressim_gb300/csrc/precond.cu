@@ -13,7 +13,6 @@
 
 #include <algorithm>
 #include <atomic>
-#include <mutex>
 #include <cstdlib>
 #include <future>
 #include <string>
@@ -789,38 +788,14 @@ static void plan_values(Context& ctx, SweepPlan& P, const double* csr_vals, bool
 
 // Cluster launch of a level walk; falls back to one launch per level when
 // clusters of the requested size cannot be scheduled.
-// Probes run once per process; contexts driven from several host threads
-// (ensembles) take the lock for them.
-static std::mutex g_probe_mu;
-static std::atomic<int> g_cluster_ok{-1};  // probed once per process
+static std::atomic<int> g_cluster_ok{-1};  // the last device's answer (rsg_sweep_mode)
 
 template <typename Kernel, typename Args>
 static bool launch_cluster(Context& ctx, const char* name, Kernel kern, const Args& args, int threads = 512) {
-  std::atomic<int>& cluster_ok = g_cluster_ok;
-  std::unique_lock<std::mutex> lk(g_probe_mu, std::defer_lock);
-  if (cluster_ok < 0) lk.lock();
-  if (cluster_ok < 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ctx.cluster_size);
-    cfg.blockDim = dim3(threads);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctx.cluster_size;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, (const void*)kern, &cfg);
-    cluster_ok = (e == cudaSuccess && nclusters >= 1) ? 1 : 0;
-    cudaGetLastError();
-  }
-  if (lk.owns_lock()) lk.unlock();
-  if (!cluster_ok) return false;
+  static PerDevice cluster_ok;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctx.cluster_size);
   cfg.blockDim = dim3(threads);
-  cfg.stream = ctx.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ctx.cluster_size;
@@ -828,6 +803,15 @@ static bool launch_cluster(Context& ctx, const char* name, Kernel kern, const Ar
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  const bool ok = cluster_ok.ask(ctx.device, [&] {
+    int nclusters = 0;
+    cudaError_t e = cudaOccupancyMaxActiveClusters(&nclusters, (const void*)kern, &cfg);
+    cudaGetLastError();
+    g_cluster_ok = e == cudaSuccess && nclusters >= 1;
+    return e == cudaSuccess && nclusters >= 1;
+  });
+  if (!ok) return false;
+  cfg.stream = ctx.stream;
   LaunchScope scope(ctx, name);
   RSG_CUDA(cudaLaunchKernelEx(&cfg, kern, args));
   return true;
@@ -874,12 +858,8 @@ static bool ring_schedulable(Kernel kern, int ctas, size_t smem) {
 template <int KIND, typename T, int CTAS, int MAXW, bool FMA>
 static bool launch_ring_n(Context& ctx, const char* name, const RingPlan& G, const RingVals<T>& a, size_t smem) {
   auto kern = k_sweep_ring<KIND, T, MAXW, CTAS, FMA>;
-  static std::atomic<int> ok{0};  // per instantiation: 0 not probed, 1 schedulable, -1 not
-  if (!ok) {
-    std::lock_guard<std::mutex> lk(g_probe_mu);
-    if (!ok) ok = ring_schedulable(kern, CTAS, RING_SMEM_MAX) ? 1 : -1;
-  }
-  if (ok < 0) return false;
+  static PerDevice ok;
+  if (!ok.ask(ctx.device, [&] { return ring_schedulable(kern, CTAS, RING_SMEM_MAX); })) return false;
   RingArgs g{G.nlev,        G.R,           G.slack,       G.slice_base.get(), G.row.get(), G.len.get(),
              G.ridx.get(), G.pmask.get(), G.expect.get(), G.nbr.get(),       ctx.dev_err.get()};
   cudaLaunchConfig_t cfg = {};

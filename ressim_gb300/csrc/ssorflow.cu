@@ -24,8 +24,6 @@
 // cluster with a barrier per level.  That solve with its setup: 58 ms (72 with
 // the ordered sums) against 285; 49 with the V-cycle's 34 kernels launched as a
 // chain, a sweep readying its shared memory beside the end of the kernel before.
-#include <mutex>
-
 #include "dataflow.cuh"
 #include "ssorflow.cuh"
 
@@ -331,17 +329,10 @@ const float* plan_val(const SweepPlan& P, float) { return P.valf.get(); }
 const double* plan_diag(const SweepPlan& P, double) { return P.diag.get(); }
 const float* plan_diag(const SweepPlan& P, float) { return P.diagf.get(); }
 
-template <typename Kernel>
-void flow_smem(std::once_flag& once, Kernel kern) {
-  std::call_once(once, [&] {
-    RSG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FLOW_SMEM));
-  });
-}
-
 template <typename T, bool BWD>
 void launch_slices(Context& ctx, const char* name, const SsorArgs<T>& a) {
-  static std::once_flag once;
-  flow_smem(once, k_ssor_slices<T, BWD>);
+  static PerDevice allowed;
+  allow_smem(allowed, ctx, k_ssor_slices<T, BWD>, FLOW_SMEM);
   launch_chained(ctx, name, k_ssor_slices<T, BWD>, 1, FLOW_THREADS<T>, sizeof(T) * a.n, a);
 }
 
