@@ -798,7 +798,9 @@ __global__ void __launch_bounds__(BW_THREADS, 1) k_block_walk(BlockWalkArgs g, B
 // 0 a scaled coefficient is not finite, bit 1 not finite in single precision.
 template <typename T, bool UPPER>
 __global__ void k_block_walk_values(int nslots, int W, const int* __restrict__ rows, const int* __restrict__ src, const double* __restrict__ lu,
-                                    const int* __restrict__ diag, T* __restrict__ out, int* __restrict__ flag) {
+                                    const int* __restrict__ diag, T* __restrict__ out, int* __restrict__ flag,
+                                    const int* __restrict__ failed, const int* __restrict__ err) {
+  if ((failed && *failed) || *err) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nslots) return;
   const int s = t >> 5, lane = t & 31;
@@ -894,14 +896,14 @@ template <>
 BlockWalkData<float>& BlockWalkPair::data<float>() { return d32; }
 
 template <typename T>
-void BlockWalkPair::values(const double* lu, const int* diag, int* flag) {
+void BlockWalkPair::values(const double* lu, const int* diag, int* flag, const int* failed) {
   BlockWalkData<T>& d = data<T>();
   d.lval.resize(std::max<size_t>(L.slots() * L.w.total(), 1));
   d.uval.resize(U.slots() * (U.w.total() + 1));
   RSG_LAUNCH(*ctx, "walk_values", (k_block_walk_values<T, false>), blocks_for(L.slots(), 256), 256, 0, (int)L.slots(),
-             L.w.total(), L.rows.get(), L.src.get(), lu, diag, d.lval.get(), flag);
+             L.w.total(), L.rows.get(), L.src.get(), lu, diag, d.lval.get(), flag, failed, ctx->dev_err.get());
   RSG_LAUNCH(*ctx, "walk_values", (k_block_walk_values<T, true>), blocks_for(U.slots(), 256), 256, 0, (int)U.slots(),
-             U.w.total(), U.rows.get(), U.src.get(), lu, diag, d.uval.get(), flag);
+             U.w.total(), U.rows.get(), U.src.get(), lu, diag, d.uval.get(), flag, failed, ctx->dev_err.get());
 }
 
 template <typename T>
@@ -931,8 +933,8 @@ void BlockWalkPair::apply(const T* b, T* x, const int* active) {
   else launch<T, true, BW_STAGES_MIN>(*ctx, uname, U, io);
 }
 
-template void BlockWalkPair::values<double>(const double*, const int*, int*);
-template void BlockWalkPair::values<float>(const double*, const int*, int*);
+template void BlockWalkPair::values<double>(const double*, const int*, int*, const int*);
+template void BlockWalkPair::values<float>(const double*, const int*, int*, const int*);
 template void BlockWalkPair::begin<double>();
 template void BlockWalkPair::begin<float>();
 template void BlockWalkPair::apply<double>(const double*, double*, const int*);

@@ -134,9 +134,10 @@ struct BlockWalkPair {
   void plan(Context* c, int n, const HostBlockWalk& lower, const HostBlockWalk& upper);
   // Gathers the coefficients from the factor values.  flag (may be null): bit
   // 0 is set when a scaled upper coefficient is not finite, bit 1 when it is
-  // not in single precision.
+  // not in single precision.  The earlier coefficients stay when the
+  // factorisation has set *failed (may be null) or a wait of it ran out.
   template <typename T>
-  void values(const double* lu, const int* diag, int* flag);
+  void values(const double* lu, const int* diag, int* flag, const int* failed = nullptr);
   // Readies the exchange arrays; once before a solve's applies (an apply
   // leaves them ready for the next one, unless it was given up).
   template <typename T>

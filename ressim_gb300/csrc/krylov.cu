@@ -931,7 +931,12 @@ SolverPtr make_solver(Context* ctx, int method, int precond, double rtol, double
 void solver_forget_matrix(Solver& s) { s.setup_for = nullptr; }
 
 void solver_setup(Solver& s, Csr& A) {
-  s.pc->setup(A);
+  try {
+    s.pc->setup(A);
+  } catch (...) {
+    if (!s.pc->serves(s.setup_for)) s.setup_for = nullptr;
+    throw;
+  }
   s.setup_for = &A;
 }
 
@@ -1030,10 +1035,7 @@ rsg_status rsg_solver_walk_shapes(rsg_solver* s, int32_t* shapes) {
 
 rsg_status rsg_solver_setup(rsg_solver* s, rsg_csr* A) {
   if (!s || !A) return RSG_BAD_ARG;
-  return guarded(s->s->ctx, [&] {
-    s->s->pc->setup(A->m);
-    s->s->setup_for = &A->m;
-  });
+  return guarded(s->s->ctx, [&] { rsg::solver_setup(*s->s, A->m); });
 }
 
 rsg_status rsg_solver_solve_device(rsg_solver* s, rsg_csr* A, const double* d_b, double* d_x, rsg_solve_info* info) {

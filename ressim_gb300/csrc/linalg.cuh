@@ -110,6 +110,8 @@ struct Precond {
   // x := M^{-1} b (x may be read as the starting iterate, as SSOR does)
   virtual void apply(const double* b, double* x, const int* active) = 0;
   virtual void trans_apply(const double* b, double* x, const int* active) = 0;
+  // whether it is (after a set-up that failed: still) that of this matrix
+  virtual bool serves(const Csr* M) const { return true; }
   // From now on its work goes to this context's stream (ILU(0) only; what was
   // queued on the other has ended).
   virtual void use(Context* c) {}

@@ -944,13 +944,14 @@ struct ILUPrecond : Precond {
   BlockWalkPair walk;
   bool walk64 = false, walk32 = false, walk32_filled = false;
   bool level64 = false, level32 = false;  // the level walks' copies hold the current factors
-  DeviceBuffer<double> LU, y;
+  DeviceBuffer<double> LU, next, y;  // next: factors being made; a set-up that fails leaves LU
   DeviceBuffer<float> yf;
   RowFactor rows;
   DeviceBuffer<int> flag, upd_ptr, upd_l, upd_j;
   const int* pattern_id = nullptr;
   explicit ILUPrecond(Context* c) : ctx(c) {}
   void use(Context* c) override { ctx = walk.ctx = c; }
+  bool serves(const Csr* M) const override { return M == A; }
 
   // elimination program of the level-by-level factorisation (see FactorArgs)
   void elimination_program(Csr& M) {
@@ -1027,6 +1028,7 @@ struct ILUPrecond : Precond {
           }
       }
     }
+    A = nullptr;  // what it was prepared for goes
     build_plan(M, Lp, false, 0, false);
     build_plan(M, Up, true, 1, true);
     if (!rows.plan(M, Lp.h_order)) elimination_program(M);
@@ -1037,6 +1039,7 @@ struct ILUPrecond : Precond {
     const HostBlockWalk wl = walks[0].get(), wu = walks[1].get();
     walk.plan(ctx, M.n, wl, wu);
     LU.resize(std::max(M.nnz, 1));
+    next.resize(std::max(M.nnz, 1));
     y.resize(M.n);
     yf.resize(M.n);
     flag.resize(2);
@@ -1060,9 +1063,9 @@ struct ILUPrecond : Precond {
   }
 
   void factor_levels(Csr& M) {
-    RSG_LAUNCH(*ctx, "ilu_copy", k_copy, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, M.val.get(), LU.get());
+    RSG_LAUNCH(*ctx, "ilu_copy", k_copy, blocks_for(M.nnz, 256), 256, 0, (int64_t)M.nnz, M.val.get(), next.get());
     FactorArgs fa{Lp.nlev,      Lp.level_slices.get(), Lp.row.get(), M.rowptr.get(), M.col.get(), M.diag.get(),
-                  upd_ptr.get(), upd_l.get(),           upd_j.get(),  LU.get(),       flag.get()};
+                  upd_ptr.get(), upd_l.get(),           upd_j.get(),  next.get(),     flag.get()};
     if (!launch_cluster(*ctx, "ilu_factor", k_factor_cluster, fa)) {
       for (int l = 0; l < Lp.nlev; ++l) {
         int slots = (Lp.h_level_slices[l + 1] - Lp.h_level_slices[l]) * 32;
@@ -1079,16 +1082,17 @@ struct ILUPrecond : Precond {
     }
     // LU.set(A) then factor() (ILU.java:80-125)
     RSG_CUDA(cudaMemsetAsync(flag.get(), 0, 2 * sizeof(int), ctx->stream));
-    if (rows.planned) rows.run(M, LU.get(), flag.get());
+    if (rows.planned) rows.run(M, next.get(), flag.get());
     else factor_levels(M);
-    level64 = level32 = walk32_filled = false;
-    if (walk.planned) walk.values<double>(LU.get(), M.diag.get(), flag.get() + 1);
+    if (walk.planned) walk.values<double>(next.get(), M.diag.get(), flag.get() + 1, flag.get());
     int h[3] = {0, 0, 0};
     RSG_CUDA(cudaMemcpyAsync(h, flag.get(), 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     RSG_CUDA(cudaMemcpyAsync(h + 2, ctx->dev_err.get(), sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     ctx->sync();
     if (h[2]) ctx->check_device_error();  // a wait between rows ran out
     if (h[0]) throw Error(RSG_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(h[0]));
+    std::swap(LU, next);
+    level64 = level32 = walk32_filled = false;
     // a factor whose scaled rows overflow keeps the level walks, which divide last
     walk64 = walk.planned && !(h[1] & 1);
     walk32 = walk.planned && !(h[1] & 2);
