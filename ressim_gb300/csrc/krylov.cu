@@ -18,7 +18,6 @@ namespace rsg {
 
 void launch_spmv_add(Context& ctx, Csr& A, double alpha, const double* x, double* y, const int* active);
 void set_ssor_params(Precond* p, double wf, double wr, int reverse);
-void release_trans_plan(const Precond* p);
 
 namespace {
 
@@ -661,7 +660,6 @@ struct Solver {
   }
   ~Solver() {
     if (hstate) cudaFreeHost(hstate);
-    release_trans_plan(pc.get());
   }
 
   void ensure(int n_) {

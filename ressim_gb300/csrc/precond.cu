@@ -935,6 +935,15 @@ static void run_sweep(Context& ctx, const char* name, const SweepPlan& P, const 
 }
 
 // ------------------------------------------------------------------ ILU ----
+// transApply (ILU.java:72-78) via column-oriented sweeps over the transpose;
+// built lazily on first use.
+struct TransPlan {
+  Csr At;
+  DeviceBuffer<int> tsrc;
+  SweepPlan Lt, Ut;
+  bool built = false;
+};
+
 struct ILUPrecond : Precond {
   Context* ctx;
   Csr* A = nullptr;
@@ -947,6 +956,7 @@ struct ILUPrecond : Precond {
   DeviceBuffer<double> LU, next, y;  // next: factors being made; a set-up that fails leaves LU
   DeviceBuffer<float> yf;
   RowFactor rows;
+  std::unique_ptr<TransPlan> trans;
   DeviceBuffer<int> flag, upd_ptr, upd_l, upd_j;
   const int* pattern_id = nullptr;
   explicit ILUPrecond(Context* c) : ctx(c) {}
@@ -1029,6 +1039,7 @@ struct ILUPrecond : Precond {
       }
     }
     A = nullptr;  // what it was prepared for goes
+    trans.reset();
     build_plan(M, Lp, false, 0, false);
     build_plan(M, Up, true, 1, true);
     if (!rows.plan(M, Lp.h_order)) elimination_program(M);
@@ -1207,16 +1218,6 @@ struct ILUPrecond : Precond {
   void trans_apply(const double* b, double* x, const int* active) override;
 };
 
-// transApply (ILU.java:72-78) via column-oriented sweeps over the transpose;
-// built lazily on first use.
-struct TransPlan {
-  Csr At;
-  DeviceBuffer<int> tsrc;
-  SweepPlan Lt, Ut;
-  bool built = false;
-};
-static std::map<const ILUPrecond*, std::unique_ptr<TransPlan>> g_trans;
-
 __global__ void k_gather_vals(int64_t n, const int* __restrict__ src, const double* __restrict__ v,
                               double* __restrict__ out) {
   int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1229,9 +1230,8 @@ __global__ void k_gather_vals(int64_t n, const int* __restrict__ src, const doub
 // UnitLowerCompRowMatrix.java:69-86) subtract the same products in row
 // order of U and L; the transposed gather subtracts them in the same order.
 void ILUPrecond::trans_apply(const double* b, double* x, const int* active) {
-  auto& tp = g_trans[this];
-  if (!tp) tp.reset(new TransPlan());
-  TransPlan& T = *tp;
+  if (!trans) trans.reset(new TransPlan());
+  TransPlan& T = *trans;
   Csr& M = *A;
   if (!T.built) {
     std::vector<int> tptr(M.n + 1, 0), tcol(M.nnz), tsrc(M.nnz);
@@ -1411,11 +1411,6 @@ void set_ssor_params(Precond* p, double wf, double wr, int reverse) {
   s->omegaF = wf;
   s->omegaR = wr;
   s->reverse = reverse != 0;
-}
-
-void release_trans_plan(const Precond* p) {
-  auto* ilu = dynamic_cast<const ILUPrecond*>(p);
-  if (ilu) g_trans.erase(ilu);
 }
 
 }  // namespace rsg

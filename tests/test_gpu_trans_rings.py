@@ -8,7 +8,12 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
+from test_gpu_sweeps import pattern27
+
+from oracle import oracle as O
+from ressim_gb300 import abi, api
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +48,18 @@ def test_transposed_sweeps_push_their_values():
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.split() == ["mode", "2"] * 4, r.stdout
+
+
+def test_transpose_follows_the_pattern(ctx):
+    """One solver set up for one pattern after another: transApply is that of
+    the last."""
+    s = api.BiCGstab(ctx, abi.PC_ILU)
+    for dims in ((6, 5, 4), (20, 9, 3), (5, 4, 3)):
+        rp, col, val = pattern27(*dims, seed=96)
+        n = len(rp) - 1
+        A = api.CompRowMatrix(ctx, n, rp, col, val)
+        s.set_matrix(A)
+        b = np.random.Generator(np.random.PCG64(5)).standard_normal(n)
+        _, xo = O.ilu(rp, col, val, b, trans=True)
+        assert np.allclose(s.apply(b, trans=True), xo, rtol=1e-12, atol=1e-14), dims
+    s.release()
