@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <future>
 #include <string>
+#include <system_error>
 
 #include "blockwalk.cuh"
 #include "factor.cuh"
@@ -698,6 +699,19 @@ static HostRing host_ring(const Csr& A, bool upper, int shape) {
   return H;
 }
 
+// f on another host thread, or, where none is to be had, when its result is
+// asked for.
+template <class F>
+static auto apart(bool on_thread, F f) -> std::future<decltype(f())> {
+  if (on_thread) {
+    try {
+      return std::async(std::launch::async, f);
+    } catch (const std::system_error&) {
+    }
+  }
+  return std::async(std::launch::deferred, f);
+}
+
 static void upload_rings(Csr& A, SweepPlan& P, const HostRing (&H)[2], bool with_diag) {
   Context& ctx = *A.ctx;
   auto up = [&](auto& dst, const auto& v) {
@@ -1011,13 +1025,13 @@ struct ILUPrecond : Precond {
         throw Error(RSG_MISSING_DIAGONAL, "Missing diagonal entry on row " + std::to_string(k + 1));
     // The schedules are independent of one another and of the rest of the
     // analysis: other host threads plan them meanwhile (large patterns only).
-    const auto how = M.nnz > 200000 ? std::launch::async : std::launch::deferred;
+    const bool large = M.nnz > 200000;
     std::future<HostRing> rings[2][2];
     for (int u = 0; u < 2; ++u)
-      for (int v = 0; v < 2; ++v) rings[u][v] = std::async(how, [&M, u, v] { return host_ring(M, u == 1, v); });
+      for (int v = 0; v < 2; ++v) rings[u][v] = apart(large, [&M, u, v] { return host_ring(M, u == 1, v); });
     std::future<HostBlockWalk> walks[2];
     for (int u = 0; u < 2; ++u)
-      walks[u] = std::async(how, [&M, u] {
+      walks[u] = apart(large, [&M, u] {
         HostBlockWalk H;
         if (!block_walks_enabled() || !plan_block_walk(M.n, M.h_rowptr, M.h_col, M.h_diag, u == 1, H)) H.nblk = 0;
         return H;

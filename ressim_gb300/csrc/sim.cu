@@ -15,7 +15,6 @@
 #include <atomic>
 #include <map>
 #include <set>
-#include <system_error>
 #include <thread>
 #include <cstring>
 #include <limits>
@@ -2453,8 +2452,9 @@ rsg_status rsg_ensemble_step_batched(int32_t count, rsg_sim* const* sims, const 
     const size_t workers = std::min<size_t>(own.size(), std::max(1u, std::thread::hardware_concurrency()));
     std::vector<std::thread> pool;
     try {
+      pool.reserve(workers);
       for (size_t w = 1; w < workers; ++w) pool.emplace_back(work);
-    } catch (const std::system_error&) {  // no more threads: those there are take all members
+    } catch (const std::exception&) {  // no more threads: those there are take all members
     }
     work();
     for (auto& t : pool) t.join();
