@@ -182,9 +182,10 @@ rsg_status rsg_solver_solve(rsg_solver* s, rsg_csr* A, const double* b, double* 
  * The level walks of ILU(0) triangular solves (rsg_precond_apply, the batched
  * solves, and the solvers' applies on patterns without a block walk) run on
  * one thread-block cluster, planned for 16 CTAs of 4 warps and for 8 CTAs of
- * 8 warps; where the solvers use them, the first setup on a pattern times
+ * 8 warps.  Where the solvers use them, the first setup on a pattern times
  * both on the factors and keeps the faster per sweep and per precision (the
- * walk autotuner).  Every shape gives the same bits.
+ * walk autotuner); elsewhere the first six rsg_precond_apply calls take them in
+ * turn and the later ones the faster.  Every shape gives the same bits.
  * rsg_solver_set_walk_shape(s, 16 or 8) fixes the shape, 0 returns to the
  * library's choice (applied at the next rsg_solver_setup);
  * rsg_solver_walk_shapes reports the clusters: FP64 lower, upper, FP32 lower,

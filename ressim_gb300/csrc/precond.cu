@@ -1053,6 +1053,7 @@ struct ILUPrecond : Precond {
       }
     }
     A = nullptr;  // what it was prepared for goes
+    picked = false;
     trans.reset();
     build_plan(M, Lp, false, 0, false);
     build_plan(M, Up, true, 1, true);
@@ -1070,8 +1071,16 @@ struct ILUPrecond : Precond {
     flag.resize(2);
   }
 
-  // the shape asked for, or 16 CTAs, where the solvers do not run the walks and nothing is timed
+  // Where the solvers do not run the level walks, set-up times nothing: the
+  // shape asked for, or 16 CTAs until Preconditioner.apply has tried both.
+  bool picked = false;
+  int trials = 0;
+  float trial_ms[2][2];  // per sweep and shape
   void pick_shapes() {
+    if (picked) return;
+    picked = true;
+    trials = 0;
+    for (auto& s : trial_ms) s[0] = s[1] = 1e30f;
     for (SweepPlan* P : {&Lp, &Up})
       for (int v = 0; v < 2; ++v)
         if (P->rings[v].R && P->rings[v].C == (force_ctas ? force_ctas : 16)) P->pick[0] = P->pick[1] = v;
@@ -1214,11 +1223,41 @@ struct ILUPrecond : Precond {
     run_sweep<SW_ILU_LOWER, double, true>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), active);
     run_sweep<SW_ILU_UPPER, double, true>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, active);
   }
-  // Preconditioner.apply as MTJ rounds it (ILU.java:64-70)
+  // Preconditioner.apply as MTJ rounds it (ILU.java:64-70).  Its first calls on
+  // a pattern take the cluster shapes in turn, timed (a shape's first call, which
+  // loads its kernels, apart); the later ones the faster shape of each sweep.
+  // Which one it is follows from how the planes fall on the CTAs rather than
+  // from the size: 64x64x8 353 us with 8 CTAs, 375 with 16; 64x64x16 402 and
+  // 395; 96x96x24 688 and 609.
+  static constexpr int TRIALS = 6;
   void apply_exact(const double* b, double* x) override {
     level_values(false);
+    const bool trial = walk64 && walk32 && !force_ctas && trials < TRIALS;
+    const int v = trials & 1;
+    cudaEvent_t e[3] = {};
+    if (trial) {
+      for (SweepPlan* P : {&Lp, &Up})
+        if (P->rings[v].R) P->pick[0] = v;
+      for (auto& q : e) q = ctx->get_event();
+      RSG_CUDA(cudaEventRecord(e[0], ctx->stream));
+    }
     run_sweep<SW_ILU_LOWER, double>(*ctx, "ilu_lower", Lp, Lp.val.get(), nullptr, b, y.get(), nullptr);
+    if (trial) RSG_CUDA(cudaEventRecord(e[1], ctx->stream));
     run_sweep<SW_ILU_UPPER, double>(*ctx, "ilu_upper", Up, Up.val.get(), Up.diag.get(), y.get(), x, nullptr);
+    if (!trial) return;
+    RSG_CUDA(cudaEventRecord(e[2], ctx->stream));
+    RSG_CUDA(cudaEventSynchronize(e[2]));
+    for (int s = 0; s < 2; ++s) {
+      float ms = 0;
+      RSG_CUDA(cudaEventElapsedTime(&ms, e[s], e[s + 1]));
+      if (trials >= 2) trial_ms[s][v] = std::min(trial_ms[s][v], ms);
+    }
+    for (auto& q : e) ctx->event_pool.push_back(q);
+    if (++trials == TRIALS)
+      for (SweepPlan* P : {&Lp, &Up}) {
+        const float* ms = trial_ms[P == &Up];
+        if (P->rings[0].R && P->rings[1].R) P->pick[0] = ms[1] < ms[0] ? 1 : 0;
+      }
   }
   void apply_f32(const float* b, float* x, const int* active) override {
     if (walk32) {
@@ -1385,7 +1424,7 @@ bool ilu_walk_shape(Precond* p, int force, int* shapes) {
   if (!ilu) return false;
   if (force >= 0) {
     ilu->force_ctas = force;
-    ilu->Lp.tuned = ilu->Up.tuned = false;  // the next setup re-tunes
+    ilu->Lp.tuned = ilu->Up.tuned = ilu->picked = false;  // the next setup re-tunes
   }
   if (shapes) {
     const SweepPlan* P[2] = {&ilu->Lp, &ilu->Up};
