@@ -490,7 +490,8 @@ def finish(args, ctx, mesh, sim, n, world, units, dev_s, wall, launches, clk, ne
         "e2e": e2e,
         "gpu_launches": launches,
         "sweep_mode": {-1: "undecided", 0: "one launch per level", 1: "one cluster walks all levels",
-                       2: "one cluster, values pushed through distributed shared memory"}.get(
+                       2: "one cluster, values pushed through distributed shared memory",
+                       3: "row blocks over all SMs"}.get(
             api.lib().rsg_sweep_mode()),
         "roofline": roof,
         "spmv": spmv,

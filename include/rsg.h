@@ -78,12 +78,14 @@ rsg_status rsg_context_create(int32_t device, rsg_ctx** out);
 rsg_status rsg_context_destroy(rsg_ctx* ctx);
 /* Last error message recorded on the context (empty if none). */
 const char* rsg_context_last_error(rsg_ctx* ctx);
-/* How the level-scheduled triangular sweeps run in this process:
+/* How the triangular sweeps have run in this process so far (of several
+ * level walks the last in this list):
  * -1 not decided yet, 0 one launch per level, 1 one thread-block cluster
  * walking all levels with hardware cluster barriers, 2 ILU sweeps on one
  * cluster whose CTAs own contiguous row blocks and push each computed value
  * through distributed shared memory to the CTAs that read it (st.async +
- * mbarrier transaction counts, no cluster barrier per level). */
+ * mbarrier transaction counts, no cluster barrier per level); 3 block walks
+ * only (the ILU(0) solves inside the Krylov solvers). */
 int32_t rsg_sweep_mode(void);
 /* Builds on the host the distributed-shared-memory schedule of one ILU(0)
  * triangular sweep of a CSR pattern (sweep 0: the unit lower solve, 1: the

@@ -881,6 +881,9 @@ void launch(Context& ctx, const char* name, const BlockWalk& P, const BlockWalkI
 
 }  // namespace
 
+static std::atomic<bool> g_used{false};
+bool block_walks_used() { return g_used.load(std::memory_order_relaxed); }
+
 void BlockWalkPair::plan(Context* c, int n, const HostBlockWalk& hl, const HostBlockWalk& hu) {
   ctx = c;
   planned = false;
@@ -924,6 +927,7 @@ void BlockWalkPair::apply(const T* b, T* x, const int* active) {
   BlockWalkData<T>& d = data<T>();
   BlockWalkIo<T> io{d.lval.get(), b, {d.lex[0].get(), d.lex[1].get()}, d.uex.get(), x, (int)L.slots(), (int)U.slots(),
                     active};
+  if (!block_walks_used()) g_used = true;
   const bool f32 = sizeof(T) == 4;
   const char *lname = f32 ? "ilu_lower_f32" : "ilu_lower", *uname = f32 ? "ilu_upper_f32" : "ilu_upper";
   if (L.stages == BW_STAGES_MAX) launch<T, false, BW_STAGES_MAX>(*ctx, lname, L, io);

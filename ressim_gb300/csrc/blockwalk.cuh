@@ -105,6 +105,9 @@ bool plan_block_walk(int n, const std::vector<int>& rp, const std::vector<int>& 
 std::string check_block_walk(int n, const std::vector<int>& rp, const std::vector<int>& cl,
                              const std::vector<int>& dg, bool upper, const HostBlockWalk& H);
 
+// Whether this process has launched a block walk.
+bool block_walks_used();
+
 struct BlockWalk {
   bool upper = false;
   int nblk = 0, halo = 0, stages = 0, nsteps = 0;

@@ -1468,7 +1468,11 @@ void set_ssor_params(Precond* p, double wf, double wr, int reverse) {
 
 }  // namespace rsg
 
-extern "C" int32_t rsg_sweep_mode(void) { return rsg::g_ring_used.load() ? 2 : rsg::g_cluster_ok.load(); }
+extern "C" int32_t rsg_sweep_mode(void) {
+  if (rsg::g_ring_used.load()) return 2;
+  const int cluster = rsg::g_cluster_ok.load();
+  return cluster < 0 && rsg::block_walks_used() ? 3 : cluster;
+}
 
 // Builds the ring schedule of one ILU(0) sweep of a pattern on the host and
 // checks it (rsg::check_ring).  Needs no GPU.
