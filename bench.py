@@ -120,12 +120,12 @@ def build_case(args):
     return case, keep, fluid, co, srcs, init, spec
 
 
-# DRAM bytes (read + write) per launch of the ILU(0) level walks, measured by
-# one ncu capture of this workload (dram__bytes_read.sum +
+# DRAM bytes (read + write) per launch of the ILU(0) block walks, measured by
+# one ncu capture on a matrix of this workload's pattern (dram__bytes_read.sum +
 # dram__bytes_write.sum); keyed by grid size and kernel family.  ncu cannot
 # run inside the timed benchmark, so the line labels these as a capture's.
-NCU_TRAFFIC = {(128, 128, 32): {"ilu_lower": 103_740_416, "ilu_upper": 107_909_632}}
-NCU_TRAFFIC_SOURCE = "ncu capture of the same kernel on the same workload (not measured in this run)"
+NCU_TRAFFIC = {(128, 128, 32): {"ilu_lower": 145_872_128, "ilu_upper": 159_775_488}}
+NCU_TRAFFIC_SOURCE = "ncu capture of the same kernel on the same pattern (not measured in this run)"
 
 
 def config_of(args, nnz, dt):

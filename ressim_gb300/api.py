@@ -797,9 +797,9 @@ def write_matrix_market_vector(path, x):
 
 
 def ensemble_step_batched(sims, dts, precision=0):
-    """One time step of every Discretisation of `sims`: members with contexts
-    of their own on their own streams, others in lockstep with one persistent
-    launch of pressure solves per Newton iteration
+    """One time step of every Discretisation of `sims`: members whose ILU(0)
+    factors have block walks on streams of their own, others in lockstep with
+    one persistent launch of pressure solves per Newton iteration
     (rsg_ensemble_step_batched).  precision 0: FP64 BiCGstab +
     ILU(0); 1: the mixed-precision solver (FP64 flexible GMRES around FP32
     BiCGstab + FP32 ILU(0)).  Returns (per-member rsg_step_info list,

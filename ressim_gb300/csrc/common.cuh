@@ -144,8 +144,8 @@ inline bool grid_empty(const dim3& g) { return g.x == 0 || g.y == 0 || g.z == 0;
 // the last ones of the kernel before it in the stream still run, and wait
 // there (programmatic dependent launch).  An iteration of a Krylov solver is a
 // chain of 9 to 11 kernels, each idle for about 2 us at its start and end on
-// small systems: 32x32x8 two-phase step 21.6 -> 19.9 ms, 64x64 potential
-// problem 6.90 -> 6.12, 128x128x32 mixed solve 80 to 88 -> 72 to 82.
+// small systems: chained, a 32x32x8 two-phase step takes 8% less, the 64x64
+// potential problem 11%, the 128x128x32 mixed solve 8%.
 template <typename... P, typename... A>
 inline void launch_chained(Context& ctx, const char* name, void (*kernel)(P...), int grid, int block, size_t smem,
                            A&&... args) {

@@ -76,7 +76,8 @@ void Context::check_device_error() {
     const int at = *h;
     RSG_CUDA(cudaMemsetAsync(dev_err.get(), 0, sizeof(int), stream));
     sync();
-    throw Error(RSG_TIMEOUT, "a level walk's wait ran out at level " + std::to_string(at - 1));
+    // the level of a level walk, the step of a block walk, the row of a factorisation or an SSOR sweep
+    throw Error(RSG_TIMEOUT, "a wait between blocks or rows ran out (at " + std::to_string(at - 1) + ")");
   }
 }
 

@@ -1143,8 +1143,8 @@ struct ILUPrecond : Precond {
     }
   }
 
-  // Walk autotuner: the first setup on a pattern times each sweep's ring
-  // schedules (16 CTAs of 4 warps, 8 CTAs of 8 warps) on the factor values,
+  // Walk autotuner, where the solvers run the level walks: the first setup on a
+  // pattern times each sweep's ring schedules (16 CTAs of 4 warps, 8 CTAs of 8 warps) on the factor values,
   // for the FP64 and the FP32 walks as the solvers run them (FP64 with fused
   // multiply-adds), and keeps the faster per sweep and precision.  Every schedule sums each row in CSR order, so the choice
   // never changes a result bit.  force_ctas (rsg_solver_set_walk_shape)
