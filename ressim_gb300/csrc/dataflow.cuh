@@ -15,6 +15,7 @@ template <>
 struct Sentinel<double> {
   using Bits = unsigned long long;
   static constexpr Bits bits = 0xfff4dead5eed0badull;
+  static __device__ __forceinline__ Bits of(double v) { return (Bits)__double_as_longlong(v); }
   static __device__ __forceinline__ Bits guard(double v) {  // a stored value is never the sentinel
     const int hi = __double2hiint(v) == (int)(bits >> 32) ? 0x7ff80000 : __double2hiint(v);
     return (Bits)(unsigned)hi << 32 | (unsigned)__double2loint(v);

@@ -1348,8 +1348,8 @@ struct SSORPrecond : Precond {
       pattern_id = M.rowptr.get();
     }
     // FP32 copies too: the mixed-precision solver smooths its FP32 AMG levels with them
-    plan_values(*ctx, Fp, M.val.get(), true, true, true);
-    plan_values(*ctx, Bp, M.val.get(), true, true, true);
+    plan_values(*ctx, Fp, M.val.get(), true, flow.reads_plan(false, false), flow.reads_plan(false, true));
+    plan_values(*ctx, Bp, M.val.get(), true, flow.reads_plan(true, false), flow.reads_plan(true, true));
     flow.values(M.val.get());
   }
   // SSOR.java:143-194; x holds the starting iterate

@@ -5,19 +5,36 @@
 //
 // What bounds a sweep is its chain of dependent rows (about 160 on a 40 x 36 x
 // 12 grid, and nearly as many rows on the narrow coarse levels of an AMG
-// hierarchy), so the values travel by the shortest way there is:
+// hierarchy), or, where many rows are independent, the double-precision pipe,
+// which a warp instruction holds for 64 cycles whatever its active lanes.
+//
+// FP64, times of one sweep:
+//  * Rows over all SMs, a warp per row, a lane per entry, the lanes' products
+//    summed in order through shuffles; values polled through L2.  40x36x12
+//    0.34 ms, 96x96x24 1.0, against 1.5 and 7.2 level by level on an 8-CTA
+//    cluster.
+//  * Rows in one CTA, values polled in shared memory: a shorter hop, one SM.
+//    Where a level has at most four rows on average: tridiagonal 20,000 rows
+//    15.5 ms against 20.0 over all SMs, 1,000 rows in 697 levels 1.63 against
+//    1.82; at eleven rows a level the one SM takes twice as long.  Rows of more
+//    than 128 entries wait for their sums rather than for hops.
+//  * Level by level, a launch each, a thread per row: a thirty-second of the
+//    pipe's time.  Where a level has 10,000 rows or more, or there are two at
+//    most: red-black order, 1,000,000 rows of 24 entries 0.15 ms against 2.3;
+//    at 3,300 rows a level (128x128x64, seven points) rows take 1.4 ms and
+//    levels 3.3.
+//
+// FP32 sweeps are the mixed-precision solver's own:
 //  * Patterns whose vector fits shared memory and whose rows have at most 32
 //    entries: one CTA, a thread per row, a warp per slice of 32 rows of one
 //    level (the sweep plan's SELL slices).  A hop is a poll of shared memory.
 //    A warp's slices are far apart in the order, so the loads of one pass
 //    behind the chain of the slices before it.
-//  * Wider rows (Galerkin products): a warp per row, a lane per entry, the
-//    lanes' products summed in order through shuffles (FP64).  One CTA while
-//    the rows are few; all SMs, with the values polled through L2, for more.
-// FP32 sweeps are the mixed-precision solver's own and owe no order to the Java
-// loop.  There a warp's row leaves the operand that comes last (of the highest
-// level) out of the sum, adds the others by a tree while it waits for it, and
-// has one multiply-add left when it is there.
+//  * Wider rows (Galerkin products): a warp per row as above, one CTA while the
+//    rows are few.  No order is owed to the Java loop: a row leaves the operand
+//    that comes last (of the highest level) out of the sum, adds the others by
+//    a tree while it waits for it, and has one multiply-add left when it is
+//    there.
 // The V-cycle sweeps of a 40 x 36 x 12 system in FP32: 26 us on the 17,280
 // rows (slices) and 20 us on average on the three coarse levels (a warp per
 // row; 34 us with the ordered sum), against 245 us on average on one 8-CTA
@@ -34,10 +51,11 @@ namespace {
 constexpr int FLOW_WIDTH = 32;               // entries of a row held in registers (slices)
 constexpr int FLOW_GROUP = 8;                // operands polled together
 constexpr int FLOW_CHUNKS = 4;               // 32 entries each held in registers (rows)
-constexpr int FLOW_ROWS_MAX = 4096;          // rows one CTA takes a warp each: 100 instructions a row
+constexpr int FLOW_ROWS_MAX = 4096;          // FP32 rows one CTA takes a warp each: 100 instructions a row
+constexpr int FLOW_FEW = 4;                  // rows a level, on average, that one CTA takes in FP64
+constexpr int FLOW_MANY = 10000;             // rows a level, on average, from which levels are launched
 constexpr size_t FLOW_SMEM = 200 * 1024;
-template <typename T>
-constexpr int FLOW_THREADS = sizeof(T) == 4 ? 512 : 256;  // slices: two or four registers an entry
+constexpr int FLOW_SLICE_THREADS = 512;
 constexpr int FLOW_ROW_THREADS = 512;
 
 // The values being computed, in the CTA's shared memory or in global memory.
@@ -118,7 +136,7 @@ __device__ __forceinline__ void await(typename Sentinel<T>::Bits (&u)[N], const 
 }
 
 template <typename T, bool BWD>
-__global__ void __launch_bounds__(FLOW_THREADS<T>, 1) k_ssor_slices(SsorArgs<T> a) {
+__global__ void __launch_bounds__(FLOW_SLICE_THREADS, 1) k_ssor_slices(SsorArgs<T> a) {
   using S = Sentinel<T>;
   extern __shared__ __align__(16) unsigned char smem[];
   T* fresh = reinterpret_cast<T*>(smem);
@@ -168,8 +186,7 @@ __global__ void __launch_bounds__(FLOW_THREADS<T>, 1) k_ssor_slices(SsorArgs<T> 
       auto& w = u[k / FLOW_GROUP][k % FLOW_GROUP];
       w = 0;
       if (k < m.len && !(BWD ? at[k] > m.row : at[k] < m.row)) {
-        if constexpr (sizeof(T) == 8) w = (typename S::Bits)__double_as_longlong(a.old[at[k]]);
-        else w = __float_as_uint(a.old[at[k]]);
+        w = S::of(a.old[at[k]]);
         at[k] = -1;  // there already
       }
     }
@@ -310,6 +327,26 @@ __global__ void __launch_bounds__(FLOW_ROW_THREADS, 1) k_ssor_rows(SsorArgs<T> a
   }
 }
 
+// One level of a sweep, a thread per row.
+template <bool BWD>
+__global__ void __launch_bounds__(256) k_ssor_level(SsorArgs<double> a, int slice0, int slices) {
+  chain_begin();
+  if (a.active && *a.active != 0) return;
+  const int q = (blockIdx.x * blockDim.x + threadIdx.x) / 32, lane = threadIdx.x & 31;
+  if (q >= slices) return;
+  const int s = slice0 + q, slot = s * 32 + lane, row = a.row[slot];
+  if (row < 0) return;
+  const int base = a.slice_base[s] + lane, len = a.len[slot];
+  double sum = 0;
+#pragma unroll 8
+  for (int k = 0; k < len; ++k) {
+    const int c = a.scol[base + 32 * k];
+    sum += a.val[base + 32 * k] * ((BWD ? c > row : c < row) ? a.out[c] : a.old[c]);
+  }
+  const double sigma = (a.b[row] - sum) / a.diag[slot], self = a.old[row];
+  a.out[row] = self + a.omega * (sigma - self);
+}
+
 template <typename T>
 __global__ void k_flow_reset(int n, T* out, unsigned* ticket, const int* active) {
   chain_begin();
@@ -324,21 +361,43 @@ __global__ void k_flow_f32(int nnz, const double* __restrict__ a, float* __restr
   if (i < nnz) b[i] = (float)a[i];
 }
 
-const double* plan_val(const SweepPlan& P, double) { return P.val.get(); }
-const float* plan_val(const SweepPlan& P, float) { return P.valf.get(); }
-const double* plan_diag(const SweepPlan& P, double) { return P.diag.get(); }
-const float* plan_diag(const SweepPlan& P, float) { return P.diagf.get(); }
+// The slices of a sweep plan.
+template <typename T>
+void slice_args(SsorArgs<T>& a, const SweepPlan& P) {
+  if constexpr (sizeof(T) == 8) {
+    a.val = P.val.get();
+    a.diag = P.diag.get();
+  } else {
+    a.val = P.valf.get();
+    a.diag = P.diagf.get();
+  }
+  a.nslices = P.nslices;
+  a.slice_base = P.slice_base.get();
+  a.row = P.row.get();
+  a.len = P.len.get();
+  a.scol = P.col.get();
+}
 
-template <typename T, bool BWD>
-void launch_slices(Context& ctx, const char* name, const SsorArgs<T>& a) {
+template <bool BWD>
+void launch_slices(Context& ctx, const char* name, const SsorArgs<float>& a) {
   static PerDevice allowed;
-  allow_smem(allowed, ctx, k_ssor_slices<T, BWD>, FLOW_SMEM);
-  launch_chained(ctx, name, k_ssor_slices<T, BWD>, 1, FLOW_THREADS<T>, sizeof(T) * a.n, a);
+  allow_smem(allowed, ctx, k_ssor_slices<float, BWD>, FLOW_SMEM);
+  launch_chained(ctx, name, k_ssor_slices<float, BWD>, 1, FLOW_SLICE_THREADS, sizeof(float) * a.n, a);
+}
+
+template <bool BWD>
+void launch_levels(Context& ctx, const char* name, const SsorArgs<double>& a, const SweepPlan& P) {
+  for (int l = 0; l < P.nlev; ++l) {
+    const int s0 = P.h_level_slices[l], slices = P.h_level_slices[l + 1] - s0;
+    launch_chained(ctx, name, k_ssor_level<BWD>, blocks_for(slices, 8), 256, 0, a, s0, slices);
+  }
 }
 
 template <typename T, bool BWD>
-void launch_rows(Context& ctx, const char* name, const SsorArgs<T>& a) {
-  if (a.n <= FLOW_ROWS_MAX) {
+void launch_rows(Context& ctx, const char* name, const SsorArgs<T>& a, bool one) {
+  if (one) {
+    static PerDevice allowed;
+    allow_smem(allowed, ctx, k_ssor_rows<T, BWD, true>, FLOW_SMEM);
     launch_chained(ctx, name, k_ssor_rows<T, BWD, true>, 1, FLOW_ROW_THREADS, sizeof(T) * a.n, a);
     return;
   }
@@ -349,22 +408,24 @@ void launch_rows(Context& ctx, const char* name, const SsorArgs<T>& a) {
 
 }  // namespace
 
-template <typename T>
-bool SsorFlow::by_slices() const {
-  return widest <= FLOW_WIDTH && sizeof(T) * (size_t)A->n <= FLOW_SMEM;
-}
-
 void SsorFlow::plan(Csr& M, const SweepPlan& fwd, const SweepPlan& bwd) {
   ctx = M.ctx;
   A = &M;
   plans[0] = &fwd;
   plans[1] = &bwd;
-  widest = 0;
+  int widest = 0;  // longest row, without its diagonal
   for (int k = 0; k < M.n; ++k) widest = std::max(widest, M.h_rowptr[k + 1] - M.h_rowptr[k] - 1);
-  if (by_slices<double>()) return;  // then by_slices<float>() too
+  slices = widest <= FLOW_WIDTH && sizeof(float) * (size_t)M.n <= FLOW_SMEM;
+  const bool wide = widest > 32 * FLOW_CHUNKS;
   for (int u = 0; u < 2; ++u) {
+    const int64_t nlev = plans[u]->nlev;
+    levels[u] = !wide && (nlev <= 2 || M.n >= FLOW_MANY * nlev);
+    few[u] = !wide && M.n <= FLOW_FEW * nlev && sizeof(double) * (size_t)M.n <= FLOW_SMEM;
+    if (levels[u] && slices) continue;  // no sweep by rows
     const std::vector<int>& o = plans[u]->h_order;
     order[u].resize(std::max<size_t>(o.size(), 1));
+    RSG_CUDA(cudaMemcpyAsync(order[u].get(), o.data(), sizeof(int) * o.size(), cudaMemcpyHostToDevice, ctx->stream));
+    if (slices) continue;
     // the entry of the highest level of each row, of several the one nearest
     // the diagonal (on a grid it is computed last)
     std::vector<int> lev(M.n, 0), entry(std::max(M.n, 1), -1);
@@ -382,22 +443,26 @@ void SsorFlow::plan(Csr& M, const SweepPlan& fwd, const SweepPlan& bwd) {
     RSG_CUDA(cudaMemcpyAsync(newest[u].get(), entry.data(), sizeof(int) * entry.size(), cudaMemcpyHostToDevice,
                              ctx->stream));
     ctx->sync();  // entry goes out of scope
-    RSG_CUDA(cudaMemcpyAsync(order[u].get(), o.data(), sizeof(int) * o.size(), cudaMemcpyHostToDevice, ctx->stream));
   }
-  val.resize(std::max(M.nnz, 1));
-  valf.resize(std::max(M.nnz, 1));
   ticket.resize(1);
 }
 
 void SsorFlow::values(const double* csr) {
-  if (by_slices<double>()) return;
-  RSG_CUDA(cudaMemcpyAsync(val.get(), csr, sizeof(double) * A->nnz, cudaMemcpyDeviceToDevice, ctx->stream));
-  RSG_LAUNCH(*ctx, "flow_f32", k_flow_f32, blocks_for(A->nnz, 256), 256, 0, A->nnz, csr, valf.get());
+  const size_t size = std::max(A->nnz, 1);
+  if (!levels[0] || !levels[1]) {
+    val.resize(size);
+    RSG_CUDA(cudaMemcpyAsync(val.get(), csr, sizeof(double) * A->nnz, cudaMemcpyDeviceToDevice, ctx->stream));
+  }
+  if (!slices) {
+    valf.resize(size);
+    RSG_LAUNCH(*ctx, "flow_f32", k_flow_f32, blocks_for(A->nnz, 256), 256, 0, A->nnz, csr, valf.get());
+  }
 }
 
 template <typename T>
 void SsorFlow::sweep(bool backward, const T* b, const T* old, T* out, T omega, const int* active) {
-  const SweepPlan& P = *plans[backward ? 1 : 0];
+  const int u = backward ? 1 : 0;
+  const SweepPlan& P = *plans[u];
   const bool f32 = sizeof(T) == 4;
   const char* name = backward ? (f32 ? "ssor_bwd_f32" : "ssor_bwd") : (f32 ? "ssor_fwd_f32" : "ssor_fwd");
   SsorArgs<T> a{};
@@ -408,28 +473,28 @@ void SsorFlow::sweep(bool backward, const T* b, const T* old, T* out, T omega, c
   a.omega = omega;
   a.active = active;
   a.err = ctx->dev_err.get();
-  if (by_slices<T>()) {
-    a.val = plan_val(P, T());
-    a.nslices = P.nslices;
-    a.slice_base = P.slice_base.get();
-    a.row = P.row.get();
-    a.len = P.len.get();
-    a.scol = P.col.get();
-    a.diag = plan_diag(P, T());
-    if (backward) launch_slices<T, true>(*ctx, name, a);
-    else launch_slices<T, false>(*ctx, name, a);
+  if (f32 ? slices : levels[u]) {
+    slice_args(a, P);
+    if constexpr (sizeof(T) == 4) {
+      if (backward) launch_slices<true>(*ctx, name, a);
+      else launch_slices<false>(*ctx, name, a);
+    } else {
+      if (backward) launch_levels<true>(*ctx, name, a, P);
+      else launch_levels<false>(*ctx, name, a, P);
+    }
     return;
   }
   if constexpr (sizeof(T) == 8) a.val = val.get();
   else a.val = valf.get();
-  a.order = order[backward ? 1 : 0].get();
-  a.newest = newest[backward ? 1 : 0].get();
+  a.order = order[u].get();
+  a.newest = newest[u].get();
   a.rowptr = A->rowptr.get();
   a.col = A->col.get();
   a.dpos = A->diag.get();
   a.ticket = ticket.get();
-  if (backward) launch_rows<T, true>(*ctx, name, a);
-  else launch_rows<T, false>(*ctx, name, a);
+  const bool one = f32 ? a.n <= FLOW_ROWS_MAX : few[u];
+  if (backward) launch_rows<T, true>(*ctx, name, a, one);
+  else launch_rows<T, false>(*ctx, name, a, one);
 }
 
 template void SsorFlow::sweep<double>(bool, const double*, const double*, double*, double, const int*);
