@@ -1024,8 +1024,10 @@ struct ILUPrecond : Precond {
       if (M.h_diag[k] < 0)
         throw Error(RSG_MISSING_DIAGONAL, "Missing diagonal entry on row " + std::to_string(k + 1));
     // The schedules are independent of one another and of the rest of the
-    // analysis: other host threads plan them meanwhile (large patterns only).
-    const bool large = M.nnz > 200000;
+    // analysis: other host threads plan them meanwhile, unless the pattern is
+    // planned before six threads have started.  Six schedules in turn of 20,000
+    // rows in red-black order take 11 ms of a 12 ms set-up, 3.4 so.
+    const bool large = M.nnz > 5000;
     std::future<HostRing> rings[2][2];
     for (int u = 0; u < 2; ++u)
       for (int v = 0; v < 2; ++v) rings[u][v] = apart(large, [&M, u, v] { return host_ring(M, u == 1, v); });

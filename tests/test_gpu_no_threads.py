@@ -53,3 +53,29 @@ def test_no_further_threads(tmp_path):
                        env=dict(os.environ, LD_PRELOAD=shim), capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     assert int(r.stdout.split()[-1]) >= 7, r.stdout  # six schedules, and the ensemble's workers
+
+
+def test_schedules_of_middling_patterns_are_planned_apart(tmp_path):
+    """Patterns of more than 5,000 entries plan their six schedules on host
+    threads (asked for here, and denied): one after the other, those of
+    scattered columns made a first set-up three times as long."""
+    shim = str(tmp_path / "deny_threads.so")
+    subprocess.run(["gcc", "-shared", "-fPIC", "-o", shim, os.path.join(HERE, "native", "deny_threads.c"), "-ldl"],
+                   check=True)
+    script = SCRIPT[:SCRIPT.index("ctx = ")] + r"""
+ctx = api.Context(0)
+for dims in ((12, 10, 5), (30, 30, 1), (4, 4, 4)):
+    rp, col = grid(*dims)
+    A = api.CompRowMatrix(ctx, len(rp) - 1, rp, col, values(rp, col, 1))
+    s = api.BiCGstab(ctx, abi.PC_ILU)
+    before = threads.threads_denied()
+    threads.deny_threads(1)
+    s.set_matrix(A)
+    threads.deny_threads(0)
+    print(len(col), threads.threads_denied() - before)
+"""
+    r = subprocess.run([sys.executable, "-c", script.format(root=os.path.dirname(HERE), tests=HERE, shim=shim)],
+                       env=dict(os.environ, LD_PRELOAD=shim), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    got = [tuple(int(v) for v in line.split()) for line in r.stdout.splitlines()]
+    assert len(got) == 3 and all(denied == (6 if entries > 5000 else 0) for entries, denied in got), got
