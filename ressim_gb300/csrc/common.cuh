@@ -167,11 +167,14 @@ inline void launch_chained(Context& ctx, const char* name, void (*kernel)(P...),
 
 #ifdef __CUDACC__
 // Before a chained kernel's first access to global memory: waits for the
-// kernel before it to end (everything it wrote is then visible), then lets
-// the next one's blocks start, as far as there is room beside this one's.
+// kernel before it to end (everything it wrote is then visible).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel's blocks start, as far as there is room beside this
+// one's, once every block has come here or ended.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void chain_begin() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
+  chain_wait();
+  chain_next();
 }
 #endif
 
