@@ -213,7 +213,9 @@ __device__ void run_epilogue(int epi, KState* s, const double* t, double* hist, 
 // cycles whatever its active lanes, so the sums over the warps' values are
 // done for all quantities at once, a lane each, instead of one after the other
 // by a thread (and in the last block by every warp).  The state that the
-// epilogue reads is loaded before the last sums.
+// epilogue works on is fetched into shared memory before the last sums: held
+// in registers it took the kernels from about 32 to 74 (a third of the warps
+// in flight: gm_mgs on 128x128x32 25 us to 29) and made the SpMV spill.
 template <int K>
 __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, int epi, KState* s, double* hist,
                               GmresDev g, int k) {
@@ -245,8 +247,10 @@ __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, in
   __syncthreads();
   if (!last) return;
   __threadfence();
-  KState c;
-  if (threadIdx.x == 0) c = *s;
+  constexpr int WORDS = sizeof(KState) / sizeof(unsigned);
+  static_assert(sizeof(KState) % sizeof(unsigned) == 0 && WORDS <= RT, "the state in words, one a thread");
+  __shared__ __align__(16) unsigned c[WORDS];
+  if (threadIdx.x < WORDS) c[threadIdx.x] = reinterpret_cast<const unsigned*>(s)[threadIdx.x];
 #pragma unroll
   for (int q = 0; q < K; ++q) {
     double x = 0;
@@ -261,9 +265,10 @@ __device__ void reduce_finish(double (&v)[K], double* part, unsigned* ticket, in
   for (int q = 0; q < K; ++q) t[q] = __shfl_sync(0xffffffffu, mine, q);
   if (lane == 0) {
     *ticket = 0;
-    run_epilogue(epi, &c, t, hist, g, k);
-    *s = c;
+    run_epilogue(epi, reinterpret_cast<KState*>(c), t, hist, g, k);
   }
+  __syncwarp();
+  for (int q = lane; q < WORDS; q += 32) reinterpret_cast<unsigned*>(s)[q] = c[q];
 }
 
 struct RedArgs {
@@ -278,7 +283,7 @@ __device__ __forceinline__ bool stopped(const KState* s) { return *(volatile con
 
 // r = b + (-1) A x (r.set(b); A.multAdd(-1, x, r)), optionally rt = r;
 // reduces r.r and r.rt.
-__global__ void __launch_bounds__(RT) k_resid(int n, const int* __restrict__ sb, const int* __restrict__ rl,
+__global__ void __launch_bounds__(RT, 8) k_resid(int n, const int* __restrict__ sb, const int* __restrict__ rl,
                                               const int* __restrict__ col, const double* __restrict__ val,
                                               const double* __restrict__ x, const double* __restrict__ b,
                                               double* __restrict__ r, double* __restrict__ rt, RedArgs ra, int epi) {
@@ -339,7 +344,7 @@ __global__ void __launch_bounds__(RT, 8) k_spmv_dot(int n, const int* __restrict
 }
 
 // Generic dot a.b
-__global__ void __launch_bounds__(RT) k_dot(int n, const double* __restrict__ a, const double* __restrict__ b,
+__global__ void __launch_bounds__(RT, 6) k_dot(int n, const double* __restrict__ a, const double* __restrict__ b,
                                             RedArgs ra, int epi, int k) {
   chain_wait();
   if (stopped(ra.s)) return;
@@ -458,7 +463,7 @@ __global__ void __launch_bounds__(RT) k_cg_update(int n, const double* __restric
 
 // ---- GMRES steps
 // w += -H(k-1,i) v_{k-1} (when k > 0), then reduce w.v_k (k <= i) or w.w (k = i+1)
-__global__ void __launch_bounds__(RT) k_gm_mgs(int n, double* __restrict__ w, const double* __restrict__ vprev,
+__global__ void __launch_bounds__(RT, 6) k_gm_mgs(int n, double* __restrict__ w, const double* __restrict__ vprev,
                                                const double* __restrict__ vk, RedArgs ra, int k, int epi) {
   chain_wait();
   if (stopped(ra.s)) return;
