@@ -140,11 +140,11 @@ inline bool grid_empty(const dim3& g) { return g.x == 0 || g.y == 0 || g.z == 0;
     ::rsg::check_launch(name);                                                   \
   } while (0)
 
-// Launch of a kernel that begins with chain_begin(): its blocks may start while
-// the last ones of the kernel before it in the stream still run, and wait
-// there (programmatic dependent launch).  An iteration of a Krylov solver is a
-// chain of 9 to 11 kernels, each idle for about 2 us at its start and end on
-// small systems: chained, a 32x32x8 two-phase step takes 8% less, the 64x64
+// Launch of a kernel that begins with chain_begin() or chain_wait(): its blocks
+// may start while the last ones of the kernel before it in the stream still run,
+// and wait there (programmatic dependent launch).  An iteration of a Krylov
+// solver is a chain of 9 to 11 kernels, each idle for about 2 us at its start and
+// end on small systems: chained, a 32x32x8 two-phase step takes 8% less, the 64x64
 // potential problem 11%, the 128x128x32 mixed solve 8%.
 template <typename... P, typename... A>
 inline void launch_chained(Context& ctx, const char* name, void (*kernel)(P...), int grid, int block, size_t smem,
@@ -172,6 +172,9 @@ __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait
 // Lets the next kernel's blocks start, as far as there is room beside this
 // one's, once every block has come here or ended.
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+// Both at once, for kernels of few blocks or of one a SM, beside which the next
+// kernel's blocks spread over the SMs, and for the V-cycle's, whose next kernel
+// is mostly a sweep of one CTA.  Others call chain_next() late (krylov.cu).
 __device__ __forceinline__ void chain_begin() {
   chain_wait();
   chain_next();
